@@ -341,7 +341,14 @@ cudaError_t launch_stencil_mt(const StencilArgs& sa, int n_st, int grid, int max
 int stencil_mt_blocks_per_sm(int max_nl, int large);  // 4 CUtensorMap per (member, pass)
 cudaError_t gemm_tc_encode(const MemberDev& M, int pass, const void* a_plane, int64_t a_plane_elems, int prec,
                            void* out);
-cudaError_t launch_gemm_simt(const GemmArgs& g, int ntiles, cudaStream_t s, bool pdl);
+// FP32 CUDA-core passes (qg_gemm_simt.cu): tile shapes, from the largest to the smallest; a
+// pass over members with N columns has simt_row_tiles(shape, rows) x simt_col_tiles(shape, N)
+// tiles of one.
+constexpr int kSimtShapes = 5;
+int simt_row_tiles(int shape, int rows);
+int simt_col_tiles(int shape, int n);
+int simt_shape(const int64_t (&tiles)[kSimtShapes], int n_sm);
+cudaError_t launch_gemm_simt(const GemmArgs& g, int shape, int ntiles, cudaStream_t s, bool pdl);
 
 // masked basins: host construction (qg_capacitance.cu) and the device correction (qg_mask.cu)
 struct CapItem {
@@ -425,7 +432,5 @@ int round_up(int v, int m);
 
 // stencil tile shapes (cells): small grids use 32 x 8, large ones 64 x 16
 constexpr int kTileSX = 32, kTileSY = 8, kTileLX = 64, kTileLY = 16;
-constexpr int kSimtBM = 64;
-constexpr int kSimtBN = 64;
 
 }  // namespace qg

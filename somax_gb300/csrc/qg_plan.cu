@@ -258,6 +258,7 @@ struct qg_plan {
     GemmTile* gy_v[5] = {};
     int n_gx_v[5] = {}, n_gy_v[5] = {};
     int n_bn = 1, bn_sel = 0;
+    int simt_sel = 0;  // tile shape of the FP32 passes
     float tune_gemm_ms[5] = {-1.f, -1.f, -1.f, -1.f, -1.f};
     // cluster-resident stepping (qg_cluster.cu): CTAs per member's cluster (0: not possible),
     // its dynamic shared memory, the members' layer count, whether qg_step uses it, and the
@@ -438,7 +439,7 @@ std::vector<GemmTile> schedule_tiles(const std::vector<GemmTile>& in, int G, con
 cudaError_t run_gemm(qg_plan* p, const GemmArgs& g, cudaStream_t s) {
     const int nt = pass_xin(g.pass) ? p->n_gx : p->n_gy;
     return timed(p, QG_K_GEMM, s, [&] {
-        if (p->opts.dst_precision == QG_DST_FP32) return launch_gemm_simt(g, nt, s, use_pdl(p));
+        if (p->opts.dst_precision == QG_DST_FP32) return launch_gemm_simt(g, p->simt_sel, nt, s, use_pdl(p));
         PersistArgs a = p->pa;
         a.g4_accumulate = g.accumulate;
         const int grid = std::max(1, std::min(nt, p->n_sm));
@@ -934,7 +935,21 @@ int qg_plan_create(const qg_member_desc* members, int n_members, const qg_option
     int64_t off_state = 0, off_x = 0, off_y = 0, off_layer = 0;
     std::vector<StencilTile> st;
     const bool tc = o.dst_precision != QG_DST_FP32;
-    const int BMg = tc ? 128 : kSimtBM;
+    // one tile shape of the FP32 passes for the plan, from the tiles of all members (the pass
+    // direction with fewer of them)
+    if (!tc) {
+        int64_t tiles[kSimtShapes];
+        for (int k = 0; k < kSimtShapes; ++k) {
+            int64_t x = 0, y = 0;
+            for (int i = 0; i < n_members; ++i) {
+                const int Ny = members[i].ny + 2, Nx = members[i].nx + 2, n = members[i].n_layers;
+                x += (int64_t)simt_row_tiles(k, n * Ny) * simt_col_tiles(k, Nx);
+                y += (int64_t)simt_row_tiles(k, n * Nx) * simt_col_tiles(k, Ny);
+            }
+            tiles[k] = std::min(x, y);
+        }
+        p->simt_sel = simt_shape(tiles, std::max(p->n_sm, 1));
+    }
     const int n_bn = tc ? kNumBN : 1;
     std::vector<GemmTile> gxv[kNumBN], gyv[kNumBN];
     std::map<long long, std::pair<float*, uint16_t*>> dst_cache;  // (size, pitch) -> device DST-I matrix
@@ -1070,11 +1085,14 @@ int qg_plan_create(const qg_member_desc* members, int n_members, const qg_option
                 for (int tx = 0; tx < (M.Nx + TX - 1) / TX; ++tx) st_v[v].push_back({i, ty, tx});
         }
         for (int v = 0; v < n_bn; ++v) {
-            const int BNg = tc ? kGemmBN[v] : kSimtBN;
-            for (int mt = 0; mt < (n * M.Ny + BMg - 1) / BMg; ++mt)
-                for (int nt = 0; nt < (M.Nx + BNg - 1) / BNg; ++nt) gxv[v].push_back({i, mt, nt});
-            for (int mt = 0; mt < (n * M.Nx + BMg - 1) / BMg; ++mt)
-                for (int nt = 0; nt < (M.Ny + BNg - 1) / BNg; ++nt) gyv[v].push_back({i, mt, nt});
+            auto rows = [&](int r) { return tc ? (r + 127) / 128 : simt_row_tiles(p->simt_sel, r); };
+            auto cols = [&](int N) {
+                return tc ? (N + kGemmBN[v] - 1) / kGemmBN[v] : simt_col_tiles(p->simt_sel, N);
+            };
+            for (int mt = 0; mt < rows(n * M.Ny); ++mt)
+                for (int nt = 0; nt < cols(M.Nx); ++nt) gxv[v].push_back({i, mt, nt});
+            for (int mt = 0; mt < rows(n * M.Nx); ++mt)
+                for (int nt = 0; nt < cols(M.Ny); ++nt) gyv[v].push_back({i, mt, nt});
         }
     }
     if (e == cudaSuccess) {
@@ -1177,7 +1195,7 @@ int qg_plan_create(const qg_member_desc* members, int n_members, const qg_option
         a.gy = p->gy_tiles;
         a.n_gx = p->n_gx;
         a.n_gy = p->n_gy;
-        a.tile_n = tc ? kGemmBN[0] : kSimtBN;
+        a.tile_n = kGemmBN[0];
         a.max_nl = p->max_nl;
         a.tc_maps = p->tc_maps;
         a.XA = p->XA;
@@ -1704,7 +1722,7 @@ int qg_plan_tuning(const qg_plan* p, int* variant, float* ms, int n) {
 
 int qg_plan_gemm_tuning(const qg_plan* p, int* tile_n, float* ms, int n) {
     if (!p) return QG_ERR_NULL;
-    if (tile_n) *tile_n = p->opts.dst_precision == QG_DST_FP32 ? kSimtBN : kGemmBN[p->bn_sel];
+    if (tile_n) *tile_n = p->opts.dst_precision == QG_DST_FP32 ? 64 : kGemmBN[p->bn_sel];
     for (int k = 0; ms && k < n && k < kNumBN; ++k) ms[k] = p->tune_gemm_ms[k];
     return QG_OK;
 }

@@ -28,6 +28,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -168,8 +169,13 @@ extern "C" int qg_invert_static(const qg_member_desc* member, const float* q, fl
     if (Nx > kStaticMaxN || Ny > kStaticMaxN) return QG_ERR_TOO_LARGE;
     if ((int64_t)nl * Ny * Px > kStaticPlane || (int64_t)nl * Nx * Py > kStaticPlane) return QG_ERR_TOO_LARGE;
     const int st_ty = (Ny + kTileSY - 1) / kTileSY, st_tx = (Nx + kTileSX - 1) / kTileSX;
-    const int gx_mt = (nl * Ny + kSimtBM - 1) / kSimtBM, gx_nt = (Nx + kSimtBN - 1) / kSimtBN;
-    const int gy_mt = (nl * Nx + kSimtBM - 1) / kSimtBM, gy_nt = (Ny + kSimtBN - 1) / kSimtBN;
+    int64_t tiles_of[kSimtShapes];
+    for (int k = 0; k < kSimtShapes; ++k)
+        tiles_of[k] = std::min((int64_t)simt_row_tiles(k, nl * Ny) * simt_col_tiles(k, Nx),
+                               (int64_t)simt_row_tiles(k, nl * Nx) * simt_col_tiles(k, Ny));
+    const int shape = simt_shape(tiles_of, 152);  // the SMs of the device this is built for
+    const int gx_mt = simt_row_tiles(shape, nl * Ny), gx_nt = simt_col_tiles(shape, Nx);
+    const int gy_mt = simt_row_tiles(shape, nl * Nx), gy_nt = simt_col_tiles(shape, Ny);
     const int n_st = st_ty * st_tx, n_gx = gx_mt * gx_nt, n_gy = gy_mt * gy_nt;
     if (n_st > kStaticMaxTiles || n_gx > kStaticMaxTiles || n_gy > kStaticMaxTiles) return QG_ERR_TOO_LARGE;
 
@@ -219,7 +225,7 @@ extern "C" int qg_invert_static(const qg_member_desc* member, const float* q, fl
         g.A = A;
         g.C = C;
         g.a_fmt = g.c_fmt = FMT_F32;
-        return launch_gemm_simt(g, nt, s, false);
+        return launch_gemm_simt(g, shape, nt, s, false);
     };
     if (!e) e = gemm(G1_FWD_X, P0, P1, gx, n_gx);
     if (!e) e = gemm(G2_FWD_Y, P1, P2, gy, n_gy);
