@@ -284,6 +284,15 @@ int qg_plan_gemm_tuning(const qg_plan* plan, int* tile_n, float* ms, int n);
    engine (-1 when not measured). */
 int qg_plan_engine(const qg_plan* plan, int* cluster_ctas, float* ms, int n);
 
+/* The row engine of qg_step (every scheme but Euler): a Runge-Kutta stage in two kernels, in FP32
+   (the x transforms and the stencil of a few rows, the y transforms of a few columns), for plans
+   whose members are alike in layers (at most 5) and grid, without land, refinement or a forced
+   variant; a tensor-core plan weighs it like the cluster engine (qg_options.cluster = 0) unless it
+   asks for the persistent kernel.  *on = 1 when the autotuner timed it faster than the
+   pass-by-pass path; *ms (may be NULL) its time of four SSP-RK3 steps (-1 when not measured).  No
+   reference counterpart. */
+int qg_plan_row_engine(const qg_plan* plan, int* on, float* ms);
+
 /* ---------------------------------------------------------------------------------------
    Multilayer shallow-water right-hand side: MultilayerShallowWater2D
    (somax/_src/models/swm/multilayer.py:150-200 vector_field, :202-219 apply_boundary_conditions,

@@ -32,6 +32,7 @@ __device__ __forceinline__ bool mbar_try(uint64_t* b, uint32_t parity) {
 }
 // Bounded wait: false after kTimeoutCycles or when another role already gave up (*abort).
 __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, volatile int* abort) {
+    if (mbar_try(b, parity)) return true;
     const long long t0 = clock64();
     while (!mbar_try(b, parity)) {
         if (abort && *abort) return false;

@@ -41,6 +41,8 @@ struct MemberDev {
     const float* Sy;        // Ny x Ny, pitch Py
     const uint16_t* Sx_bf;  // bf16 hi/lo planes of Sx (pitch Px, hi then lo), or null
     const uint16_t* Sy_bf;
+    const float4* Sx_quad;  // Sx, Sy by quads of k (the row engine), or null
+    const float4* Sy_quad;
     // masked basin (null / 0 without land)
     const uint8_t* mask;    // (Ny, Nx), 1 = ocean; interior cells with 0 are land
     int nb;                 // land boundary points B (capacitance correction)
@@ -349,6 +351,70 @@ int simt_row_tiles(int shape, int rows);
 int simt_col_tiles(int shape, int n);
 int simt_shape(const int64_t (&tiles)[kSimtShapes], int n_sm);
 cudaError_t launch_gemm_simt(const GemmArgs& g, int shape, int ntiles, cudaStream_t s, bool pdl);
+
+// FP32 row engine (qg_rows.cu) of plans whose members are alike in layers and grid: arguments of
+// its launches (one per (member, rows) or (member, mode, columns)).
+enum RowKind : int { kFirst = 0, kStage = 1 };
+// One axis of N points: half = ceil(N / 2) columns of the folded transform (nw warps of 32),
+// tn of them a lane and ng warps across; vectors padded to NP = 4 quads floats (nc warps wide);
+// the matrix passes through shared memory in nch chunks of kc quads of k (nch = 1: in one piece).
+struct RowAxis {
+    int N, half, NP, quads, nw, nc, ng, tn, kc, nch;
+    int nw_inv, nc_inv, ng_inv;  // 65536 / d + 1
+};
+// Warp groups over the rows of a transform of RC rows with TN columns a lane: a lane's
+// accumulators and operands within the 128 registers of a 512-thread CTA.
+__host__ __device__ constexpr int row_groups(int RC, int TN) {
+    return RC * TN <= 32 ? 1 : ((RC + 1) / 2 * TN <= 32 ? 2 : 4);
+}
+struct RowsArgs {
+    const MemberDev* members;
+    RowAxis x;
+    int ks_back, ks_own;  // warp groups over k of the halo rows' and of the own rows' transform
+    int Ny, Px, layers, rows, bands;  // rows: per CTA
+    int o_x, o_q, o_lap, o_op, o_s;            // shared-memory offsets (floats)
+    size_t smem;
+    const float* V;       // modal plane in: k_cols' result (kStage)
+    float* T;             // modal plane out (x transformed)
+    const float* q;       // kFirst: the state in caller packing; kStage: the stage input (x-row)
+    int zero_ring;        // kFirst: y_next's ring is zeroed
+    const float* params;
+    float* dq;            // the tendency (caller packing), or null
+    const float* y0;      // the step's state (x-row)
+    float* y_next;        // x-row: kFirst a copy of q, kStage the next stage input or the new state
+    int final_stage;
+    float a, b, dt;       // y_next = a y0 + b (q + dt dq), or with n_k > 0 the Butcher form
+    int n_k;              // stage derivatives combined, this stage's the last (0: Shu-Osher form)
+    const float* k;       // the earlier ones' caller-packed fields, kplane floats apart
+    int64_t kplane;
+    float coef[kMaxButcher];  // of the earlier ones
+    float coef_own;           // of this stage's
+    int* flags;
+};
+struct ColsArgs {
+    const MemberDev* members;
+    RowAxis x;            // the y axis
+    int ks;               // warp groups over k
+    int Nx, Px, layers, cols, nblk;  // cols: per CTA, nblk CTAs a mode
+    int o_x, o_ey, o_red, o_s;
+    size_t smem;
+    const float* T;
+    float* V;
+    int* flags;
+};
+constexpr int kRowLayers = 5;  // most layers of the row engine
+using RowsKernel = void (*)(const RowsArgs);
+using ColsKernel = void (*)(const ColsArgs);
+struct RowsTable {
+    RowsKernel rows[kRowLayers][3][2];  // by layers, rows per CTA (1, 2, 4) and kind
+    ColsKernel cols[8];
+};
+int rows_quad_floats(int N);
+void rows_quad_matrix(const float* S, int N, int ld, float* out);
+bool rows_plan(int nl, int Ny, int Nx, int n_members, int n_sm, RowsArgs* r, ColsArgs* c);
+cudaError_t rows_init(const RowsArgs& r, const ColsArgs& c);
+cudaError_t launch_rows(int kind, const RowsArgs& a, int n_members, cudaStream_t s, bool pdl);
+cudaError_t launch_cols(const ColsArgs& a, int n_members, cudaStream_t s, bool pdl);
 
 // masked basins: host construction (qg_capacitance.cu) and the device correction (qg_mask.cu)
 struct CapItem {

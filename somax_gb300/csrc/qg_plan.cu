@@ -259,6 +259,12 @@ struct qg_plan {
     int n_gx_v[5] = {}, n_gy_v[5] = {};
     int n_bn = 1, bn_sel = 0;
     int simt_sel = 0;  // tile shape of the FP32 passes
+    // FP32 row engine (qg_rows.cu): the constant part of its launches' arguments, whether the
+    // members allow it, whether the plan runs it, and the autotuner's time
+    RowsArgs rw{};
+    ColsArgs rc{};
+    bool rw_ok = false, rw_on = false;
+    float tune_rows_ms = -1.f;
     float tune_gemm_ms[5] = {-1.f, -1.f, -1.f, -1.f, -1.f};
     // cluster-resident stepping (qg_cluster.cu): CTAs per member's cluster (0: not possible),
     // its dynamic shared memory, the members' layer count, whether qg_step uses it, and the
@@ -447,6 +453,23 @@ cudaError_t run_gemm(qg_plan* p, const GemmArgs& g, cudaStream_t s) {
     });
 }
 
+RowsArgs rows_args(qg_plan* p) {
+    RowsArgs a = p->rw;
+    a.V = p->XA;
+    a.T = p->XB;
+    return a;
+}
+cudaError_t run_rows(qg_plan* p, int kind, const RowsArgs& a, cudaStream_t s) {
+    return timed(p, kind == kStage ? QG_K_STENCIL : QG_K_PREP, s,
+                 [&] { return launch_rows(kind, a, p->n_members, s, use_pdl(p)); });
+}
+// both y transforms: XB (x transformed) -> XA
+cudaError_t run_cols(qg_plan* p, cudaStream_t s) {
+    ColsArgs c = p->rc;
+    c.T = p->XB;
+    c.V = p->XA;
+    return timed(p, QG_K_GEMM, s, [&] { return launch_cols(c, p->n_members, s, use_pdl(p)); });
+}
 // psi_hat (XC) from the modal operand already in XA (and XQ for refinement).
 cudaError_t run_dst_solve(qg_plan* p, cudaStream_t s) {
     const int f = p->op_fmt;
@@ -665,10 +688,50 @@ cudaError_t run_one_step_butcher(qg_plan* p, const float* params, float dt, cons
     return e;
 }
 
+// One time step of the state in S0 with the row engine (XB holding the x-transformed modes of
+// BC(S0)): per stage the y transforms, then everything else.  Stage k reads one stage plane
+// and its neighbours' rows and writes another: S0, then S1 and S2 in turn, S0 at the end.
+cudaError_t run_one_step_rows(qg_plan* p, const float* params, float dt, int scheme, cudaStream_t s) {
+    const Tableau* tb = butcher(scheme);
+    Stage st[4];
+    const int ns = tb ? tb->n : scheme_stages(scheme, st);
+    float* const buf[2] = {p->S1, p->S2};
+    for (int k = 0; k < ns; ++k) {
+        const bool fin = k == ns - 1;
+        cudaError_t e = run_cols(p, s);
+        if (e) return e;
+        RowsArgs a = rows_args(p);
+        a.q = k == 0 ? p->S0 : buf[(k - 1) & 1];
+        a.params = params;
+        a.y0 = p->S0;
+        a.y_next = fin ? p->S0 : buf[k & 1];
+        a.final_stage = fin;
+        a.dt = dt;
+        if (tb) {
+            a.dq = p->K + (size_t)k * p->state_size;
+            a.k = p->K;
+            a.kplane = p->state_size;
+            a.n_k = k + 1;
+            for (int j = 0; j < k; ++j) a.coef[j] = (float)(fin ? tb->b[j] : tb->a[k + 1][j]);
+            a.coef_own = (float)(fin ? tb->b[k] : tb->a[k + 1][k]);
+        } else {
+            a.a = st[k].a;
+            a.b = st[k].b;
+        }
+        if ((e = run_rows(p, kStage, a, s))) return e;
+    }
+    return cudaSuccess;
+}
+
+// The row engine steps every scheme of more than one stage (a one-stage scheme would update
+// the state while its neighbours still read it).
+bool steps_in_rows(const qg_plan* p, int scheme) { return p->rw_on && scheme != QG_SCHEME_EULER; }
+
 // One time step of the state in S0 (XA holding Cl2m BC(S0)).  Stage k reads stage plane k
 // (S0, S1, S2) and writes stage plane k + 1; the final stage updates S0 in place (it reads S0
 // only pointwise there) and leaves XA ready for the next step.
 cudaError_t run_one_step(qg_plan* p, const float* params, float dt, int scheme, cudaStream_t s) {
+    if (steps_in_rows(p, scheme)) return run_one_step_rows(p, params, dt, scheme, s);
     if (const Tableau* tb = butcher(scheme)) return run_one_step_butcher(p, params, dt, *tb, s);
     Stage st[4];
     const int ns = scheme_stages(scheme, st);
@@ -768,7 +831,7 @@ cudaError_t autotune_gemm(qg_plan* p) {
     return e;
 }
 
-int autotune_engine(qg_plan* p);
+int autotune_engine(qg_plan* p, bool cluster);
 
 // Autotuner: time every stencil variant (tile shapes, sweep strip heights) in its setting,
 // one RK stage (the four DST passes, then the step-mode stencil) on the plan's own planes
@@ -953,6 +1016,20 @@ int qg_plan_create(const qg_member_desc* members, int n_members, const qg_option
     const int n_bn = tc ? kNumBN : 1;
     std::vector<GemmTile> gxv[kNumBN], gyv[kNumBN];
     std::map<long long, std::pair<float*, uint16_t*>> dst_cache;  // (size, pitch) -> device DST-I matrix
+    // the row engine: no refinement, land or forced variant, members alike in layers and grid; it
+    // computes in FP32, like the cluster engine, so that a tensor-core plan takes it under the
+    // same switch (and not when it asks for the persistent kernel)
+    std::map<int, const float4*> quad_cache;
+    p->rw_ok = (!tc || (o.cluster == 0 && !o.persistent)) && o.refine_sweeps == 0 && !o.stencil && !o.gemm_tile &&
+               n_members <= 65535;
+    for (int i = 0; i < n_members && p->rw_ok; ++i) {
+        const qg_member_desc &d = members[i], &d0 = members[0];
+        p->rw_ok = d.n_layers == d0.n_layers && d.nx == d0.nx && d.ny == d0.ny;
+        for (int j = 1; d.mask && j <= d.ny && p->rw_ok; ++j)
+            for (int k = 1; k <= d.nx && p->rw_ok; ++k) p->rw_ok = d.mask[(size_t)j * (d.nx + 2) + k] != 0;
+    }
+    p->rw_ok = p->rw_ok && rows_plan(members[0].n_layers, members[0].ny + 2, members[0].nx + 2, n_members,
+                                     std::max(p->n_sm, 1), &p->rw, &p->rc);
     for (int i = 0; i < n_members; ++i) {
         const qg_member_desc& d = members[i];
         MemberDev& M = p->mh[i];
@@ -1027,6 +1104,13 @@ int qg_plan_create(const qg_member_desc* members, int n_members, const qg_option
                     uint16_t* dbf = nullptr;
                     cudaError_t ee = upload(p, &d32, S);
                     if (!ee && o.dst_precision == QG_DST_BF16X3) ee = split(S, &dbf);
+                    if (!ee && p->rw_ok) {
+                        std::vector<float> P(rows_quad_floats(nn));
+                        rows_quad_matrix(S.data(), nn, ld, P.data());
+                        float* dp = nullptr;
+                        ee = upload(p, &dp, P);
+                        quad_cache[nn] = reinterpret_cast<const float4*>(dp);
+                    }
                     if (ee) return ee;
                     it = dst_cache.emplace(key, std::make_pair(d32, dbf)).first;
                 }
@@ -1039,6 +1123,10 @@ int qg_plan_create(const qg_member_desc* members, int n_members, const qg_option
             if ((e = shared_dst(M.Nx, M.Px, &dSx, &bx)) || (e = shared_dst(M.Ny, M.Py, &dSy, &byy))) break;
             M.Sx = dSx;
             M.Sy = dSy;
+            if (p->rw_ok) {
+                M.Sx_quad = quad_cache[M.Nx];
+                M.Sy_quad = quad_cache[M.Ny];
+            }
             M.Sx_bf = bx;
             M.Sy_bf = byy;
         }
@@ -1109,6 +1197,9 @@ int qg_plan_create(const qg_member_desc* members, int n_members, const qg_option
             p->n_st_v[v] = (int)st_v[v].size();
             e = upload(p, &p->st_tiles_v[v], st_v[v]);
         }
+        p->rw.members = p->rc.members = p->md;
+        p->rw.Px = p->rc.Px = p->mh[0].Px;
+        if (!e && p->rw_ok) e = rows_init(p->rw, p->rc);
         if (!e && !cap.empty()) {
             p->n_cap = (int)cap.size();
             e = upload(p, &p->cap_items, cap);
@@ -1189,6 +1280,7 @@ int qg_plan_create(const qg_member_desc* members, int n_members, const qg_option
         }
     }
     if (e == cudaSuccess) {
+        p->rw.flags = p->rc.flags = p->flags;
         PersistArgs& a = p->pa;
         a.members = p->md;
         a.gx = p->gx_tiles;
@@ -1248,11 +1340,17 @@ int qg_plan_create(const qg_member_desc* members, int n_members, const qg_option
             p->cl_C = cluster_size_for(p->cl_nl, members[0].ny + 2, members[0].nx + 2, &p->cl_smem);
         }
         if (p->cl_C > 0 && o.cluster == 1) p->cl_use = true;
-        // the autotuner weighs it only when no stencil variant or tile width is forced (a
-        // forced choice asks for the multi-launch path)
-        if (p->cl_C > 0 && o.cluster == 0 && o.autotune && !o.stencil && !o.gemm_tile) {
-            const int r = autotune_engine(p);
+    }
+    if (e == cudaSuccess) {
+        // the autotuner weighs the engines only when no stencil variant or tile width is forced
+        // (a forced choice asks for the pass-by-pass path); without it the row engine steps FP32
+        // plans whose members allow it
+        const bool cluster = p->cl_C > 0 && o.cluster == 0;
+        if ((cluster || p->rw_ok) && o.autotune && !o.stencil && !o.gemm_tile) {
+            const int r = autotune_engine(p, cluster);
             if (r != QG_OK) e = cudaErrorUnknown;
+        } else {
+            p->rw_on = p->rw_ok && !tc;
         }
     }
     if (e != cudaSuccess) {
@@ -1407,7 +1505,16 @@ int qg_step(qg_plan* p, float* q, const float* params, double dt, int n_steps, i
                                     cudaMemcpyDeviceToDevice, s);
     // the state lives in S0 for the whole call; its ring is zeroed only for a new
     // integration (integrate() applies the BC to state0), stage inputs always read a zero ring
-    if (!e) e = run_prep(p, q, p->S0, (flags & QG_STEP_APPLY_BC) ? 1 : 0, 1, s);
+    const int zero_ring = (flags & QG_STEP_APPLY_BC) ? 1 : 0;
+    if (!e && steps_in_rows(p, scheme)) {
+        RowsArgs a = rows_args(p);
+        a.q = q;
+        a.y_next = p->S0;
+        a.zero_ring = zero_ring;
+        e = run_rows(p, kFirst, a, s);
+    } else if (!e) {
+        e = run_prep(p, q, p->S0, zero_ring, 1, s);
+    }
     if (e) return cuda_err(e);
     // while profiling, the multi-launch path runs so that every kernel class gets its events
     const bool persistent = p->opts.persistent && p->opts.dst_precision != QG_DST_FP32 &&
@@ -1734,6 +1841,13 @@ int qg_plan_engine(const qg_plan* p, int* cluster_ctas, float* ms, int n) {
     return QG_OK;
 }
 
+int qg_plan_row_engine(const qg_plan* p, int* on, float* ms) {
+    if (!p) return QG_ERR_NULL;
+    if (on) *on = p->rw_on;
+    if (ms) *ms = p->tune_rows_ms;
+    return QG_OK;
+}
+
 int qg_set_profiling(qg_plan* p, int enable) {
     if (!p) return QG_ERR_NULL;
     cudaDeviceSynchronize();
@@ -1760,11 +1874,19 @@ int qg_kernel_stats(qg_plan* p, int k, double* total_ms, int64_t* launches) {
 
 namespace {
 
-// Autotuner: time four SSP-RK3 steps of a zero state through qg_step with the multi-launch
-// path (graph replay) and with the cluster engine, after one warm-up call each, and keep the
-// faster.  The state is the YA plane (it holds at least one packed field), the parameters
-// ones in the K planes.
-int autotune_engine(qg_plan* p) {
+void drop_step_graphs(qg_plan* p) {
+    for (cudaGraphExec_t* x : {&p->graph.exec, &p->graph.exec_k, &p->vjp_graph.exec})
+        if (*x) {
+            cudaGraphExecDestroy(*x);
+            *x = nullptr;
+        }
+}
+
+// Autotuner: time four SSP-RK3 steps of a zero state through qg_step pass by pass, with the row
+// engine (if the members allow it) and with the cluster engine (if asked to), after one
+// warm-up call each, and keep the fastest.  The state is the YA plane (it holds at least one
+// packed field), the parameters ones in the K planes.
+int autotune_engine(qg_plan* p, bool cluster) {
     cudaStream_t s = p->cap;
     float* qd = p->YA;
     float* prm = p->K;
@@ -1780,19 +1902,27 @@ int autotune_engine(qg_plan* p) {
         return QG_ERR_CUDA;
     }
     int r = QG_OK;
-    for (int use = 0; use < 2 && r == QG_OK; ++use) {
-        p->cl_use = use != 0;
+    const bool forced = p->cl_use;  // a forced cluster engine steps; the others are weighed all the same
+    float t[3] = {-1.f, -1.f, -1.f};  // pass by pass, rows, cluster
+    for (int v = 0; v < 3 && r == QG_OK; ++v) {
+        if ((v == 1 && !p->rw_ok) || (v == 2 && !cluster)) continue;
+        p->rw_on = v == 1;
+        p->cl_use = v == 2;
         r = qg_step(p, qd, prm, 1200.0, 1, QG_SCHEME_SSPRK3, 0, s);
         if (r == QG_OK && cudaEventRecord(e0, s)) r = QG_ERR_CUDA;
         if (r == QG_OK) r = qg_step(p, qd, prm, 1200.0, 4, QG_SCHEME_SSPRK3, 0, s);
-        float ms = -1.f;
-        if (r == QG_OK && (cudaEventRecord(e1, s) || cudaEventSynchronize(e1) || cudaEventElapsedTime(&ms, e0, e1)))
+        if (r == QG_OK && (cudaEventRecord(e1, s) || cudaEventSynchronize(e1) || cudaEventElapsedTime(&t[v], e0, e1)))
             r = QG_ERR_CUDA;
-        p->tune_engine_ms[use] = ms;
+        drop_step_graphs(p);
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    p->cl_use = r == QG_OK && p->tune_engine_ms[1] >= 0.f && p->tune_engine_ms[1] < p->tune_engine_ms[0];
+    p->rw_on = r == QG_OK && t[1] >= 0.f && t[1] < t[0];
+    const float multi = p->rw_on ? t[1] : t[0];
+    p->cl_use = r == QG_OK && (forced || (t[2] >= 0.f && t[2] < multi));
+    p->tune_engine_ms[0] = multi;
+    p->tune_engine_ms[1] = t[2];
+    p->tune_rows_ms = t[1];
     int flags = 0;
     if (r == QG_OK) qg_status(p, &flags, s);  // clear what the timing runs left
     return r;

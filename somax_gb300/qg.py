@@ -397,8 +397,11 @@ class Plan:
         stages = {"euler": 1, "heun": 2, "ssprk3": 3, "tsit5": 6}[scheme]
         butcher = scheme in ("euler", "tsit5")
         masked = any(m.mask is not None for m in self.members)
-        if self.engine()["cluster_ctas"] and not butcher:
+        engine = self.engine()
+        if engine["cluster_ctas"] and not butcher:
             return 1  # the cluster-resident step kernel, every stage of every step
+        if engine["rows"] and scheme != "euler":
+            return 2 + 2 * n_steps * stages  # first transform, (columns, rows) per stage, unpack
         if self.persistent and self.precision != "fp32" and self.refine == 0 and not butcher and not masked:
             return 3  # pack, the persistent step kernel, unpack
         # the column-sweep stencils launch once per distinct layer count, the layer-per-warp
@@ -437,13 +440,16 @@ class Plan:
 
     def engine(self) -> dict:
         """The stepping engine of ``step`` (Heun / SSP-RK3): the cluster size of the cluster-
-        resident engine (0: the multi-launch path) and the autotuner's time (ms) of four SSP-RK3
-        steps with each."""
+        resident engine (0: the multi-launch path), whether the multi-launch path is the FP32 row
+        engine (two kernels a stage) and the autotuner's time (ms) of four SSP-RK3 steps with each."""
         n = C.c_int()
         ms = (C.c_float * 2)()
         check(self._L.qg_plan_engine(self._h, C.byref(n), ms, 2), "qg_plan_engine")
-        return {"cluster_ctas": n.value, "ms": {"multi_launch": round(float(ms[0]), 5),
-                                                "cluster": round(float(ms[1]), 5)}}
+        on, rms = C.c_int(), C.c_float()
+        check(self._L.qg_plan_row_engine(self._h, C.byref(on), C.byref(rms)), "qg_plan_row_engine")
+        return {"cluster_ctas": n.value, "rows": bool(on.value),
+                "ms": {"multi_launch": round(float(ms[0]), 5), "cluster": round(float(ms[1]), 5),
+                       "rows": round(float(rms.value), 5)}}
 
     def set_wait_limit(self, cycles: int = 0):
         """Clock64 cycles the persistent step kernel waits at a grid barrier before it gives
