@@ -104,6 +104,7 @@ struct StageArgs {
     int ns;
     int last;             // 1: out = the next state
     int bc;               // boundary rules on read
+    float* ysave;         // SAVE: receives the stage input at the own cells (ring cells as the rules read them)
     float a[kMaxButcher];
     float b[kMaxButcher];
 };
@@ -256,7 +257,7 @@ __device__ __forceinline__ void swm_tend(const Tab& t, const SwmDev& d, int e, i
 // the derived C-grid quantities at the same points, then combines its own cell's tendencies
 // from those tables.  The own cell's state and stage derivatives stay in registers for the
 // last stage's next state.
-template <int NS, bool LAST, bool INT>
+template <int NS, bool LAST, bool SAVE, bool INT>
 __device__ __forceinline__ void stage_tile(StageTables& t, const SwmDev& d, const StageArgs& a) {
     const int tid = threadIdx.y * kSwTX + threadIdx.x;
     const int i0 = blockIdx.x * kSwTX - 1, j0 = blockIdx.y * kSwTY - 1;  // origin of the haloed tile
@@ -328,6 +329,7 @@ __device__ __forceinline__ void stage_tile(StageTables& t, const SwmDev& d, cons
                     for (int m = 0; m < NS; ++m) r = fmaf(a.b[m], ko[m], r);
                 }
                 a.out[off] = r;
+                if (SAVE) a.ysave[off] = yo3[f];
             }
         }
         __syncthreads();
@@ -344,15 +346,15 @@ __device__ __forceinline__ void stage_tile(StageTables& t, const SwmDev& d, cons
     if (bad && a.flags) atomicOr(a.flags, 1);
 }
 
-template <int NS, bool LAST>
+template <int NS, bool LAST, bool SAVE>
 __global__ void __launch_bounds__(kSwTX * kSwTY) k_swm_stage(SwmDev d, StageArgs a) {
     __shared__ StageTables t;
     const int i0 = blockIdx.x * kSwTX - 1, j0 = blockIdx.y * kSwTY - 1;
     const bool interior = i0 >= 1 && i0 + kStX - 1 <= d.Nx - 3 && j0 >= 1 && j0 + kStY - 1 <= d.Ny - 3;
     if (interior)
-        stage_tile<NS, LAST, true>(t, d, a);
+        stage_tile<NS, LAST, SAVE, true>(t, d, a);
     else
-        stage_tile<NS, LAST, false>(t, d, a);
+        stage_tile<NS, LAST, SAVE, false>(t, d, a);
 }
 
 // ---- cluster-resident engine: every step of a small basin in one thread-block cluster -----
@@ -566,222 +568,252 @@ __global__ void __launch_bounds__(kScThreads) k_swm_cluster(SwmClusterArgs a) {
 // ---- adjoint of the right-hand side --------------------------------------------------------
 //
 // The transpose of vector_field's Jacobian at a stage input Y, applied to a cotangent
-// gbar = (dh_bar, du_bar, dv_bar), as gathers in two passes:
-//  k_swm_vjp_mid  the cotangents of the intermediate quantities at every point: PV at the X
-//                 points (q_bar), the face mass fluxes of the PV flux (vh_bar at V points,
-//                 uh_bar at U points), the Bernoulli potential at T points (P_bar = ke_bar, and
-//                 the pressure sum's), and the upwind mass fluxes (Fx_bar on east faces, Fy_bar
-//                 on north faces), each gathered from the tendencies that read it;
-//  k_swm_vjp_in   the cotangent of the stage input (after the boundary rules) at every point,
-//                 gathered from those and the direct terms (Laplacians, drag); the pressure sum
-//                 sum_{l<=k} g'_l h_l becomes a reverse cumulative sum over the layers; and the
-//                 parameter cotangents (nu, kappa, tau0) summed over the grid;
-//  k_swm_bc_vjp   the transpose of the boundary rules: every ring or wall-face value that
-//                 copied a source cell passes its cotangent on to it (zeroed values drop theirs).
+// gbar = (dh_bar, du_bar, dv_bar), as gathers:
+//  k_swm_vjp      per layer and tile, in shared memory: the stage input (boundary rules on read)
+//                 and gbar with a two-cell halo, PV, face mass fluxes and layer thickness at the X
+//                 points; the cotangents of the intermediate quantities (PV at the X points, the
+//                 face mass fluxes of the PV flux, the Bernoulli potential at T points, the upwind
+//                 mass fluxes), each gathered from the tendencies that read it; and from those
+//                 and the direct terms (Laplacians, drag) the cotangent of the stage input and the
+//                 parameter cotangents.  The pressure sum sum_{l<=k} g'_l h_l becomes a sum of the
+//                 potential's cotangents over the layers k and below.
+//  k_swm_scatter  the transpose of the boundary rules (every ring or wall-face value that copied a
+//                 source cell passes its cotangent on to it, gathered at the source; zeroed values
+//                 drop theirs), added to the cotangents of the step's state and of the earlier
+//                 stage derivatives.
 // The upwind switch and the PV division are differentiated where they are smooth (the switch
 // as a constant choice of upwind cell).
+//
+// Bound: launches and latency on small basins.  Two kernels that formed every intermediate from
+// global memory at each of its readers (~200 loads a point and layer, boundary rules and all), a
+// third for the boundary rules and an axpy per stage derivative took 331 us for a Tsit5 step's
+// adjoint at 2 x 66^2, 63 launches; these take 123 us, the forward stages included (the smallest
+// tile that fills a warp's row: 18 CTAs a layer).
 
-// Forward values of the right-hand side at any point of layer k of the stage input y, with
-// the boundary rules on read when bc (the same expressions as the stage kernel's).
-struct SwmAt {
-    const SwmDev& d;
-    const float* y;
-    int64_t plane, field;
-    bool bc;
-    __device__ __forceinline__ bool inside(int a, int b) const {
-        return a >= 1 && a <= d.Ny - 2 && b >= 1 && b <= d.Nx - 2;
-    }
-    __device__ __forceinline__ float H(int k, int a, int b) const { return ld(y + k * plane, d, 0, a, b, bc); }
-    __device__ __forceinline__ float U(int k, int a, int b) const { return ld(y + field + k * plane, d, 1, a, b, bc); }
-    __device__ __forceinline__ float V(int k, int a, int b) const {
-        return ld(y + 2 * field + k * plane, d, 2, a, b, bc);
-    }
-    __device__ __forceinline__ float hX(int k, int a, int b) const {
-        return 0.25f * (H(k, a, b) + H(k, a, b + 1) + H(k, a + 1, b) + H(k, a + 1, b + 1));
-    }
-    __device__ __forceinline__ float qX(int k, int a, int b) const {
-        if (!inside(a, b)) return 0.f;
-        const float zeta = (V(k, a, b + 1) - V(k, a, b)) * d.idx - (U(k, a + 1, b) - U(k, a, b)) * d.idy;
-        return (zeta + __ldg(d.fx + a)) / hX(k, a, b);
-    }
-    __device__ __forceinline__ float uh(int k, int a, int b) const {
-        return inside(a, b) ? 0.5f * (H(k, a, b) + H(k, a, b + 1)) * U(k, a, b) : 0.f;
-    }
-    __device__ __forceinline__ float vh(int k, int a, int b) const {
-        return inside(a, b) ? 0.5f * (H(k, a, b) + H(k, a + 1, b)) * V(k, a, b) : 0.f;
-    }
-    // at an interior output cell (j, i)
-    __device__ __forceinline__ float qU(int k, int j, int i) const { return 0.5f * (qX(k, j, i) + qX(k, j - 1, i)); }
-    __device__ __forceinline__ float qV(int k, int j, int i) const { return 0.5f * (qX(k, j, i) + qX(k, j, i - 1)); }
-    __device__ __forceinline__ float vhU(int k, int j, int i) const {
-        return 0.25f * (vh(k, j, i) + vh(k, j, i + 1) + vh(k, j - 1, i) + vh(k, j - 1, i + 1));
-    }
-    __device__ __forceinline__ float uhV(int k, int j, int i) const {
-        return 0.25f * (uh(k, j, i) + uh(k, j, i - 1) + uh(k, j + 1, i) + uh(k, j + 1, i - 1));
-    }
-};
+constexpr int kVjX = 32, kVjY = 4, kVjSX = kVjX + 4, kVjSY = kVjY + 4, kVjE = kVjSX * kVjSY;
 
-// Mid-point cotangents: six planes per layer in `mid` ([k][0..5][Ny][Nx]: q_bar, vh_bar,
-// uh_bar, P_bar, Fx_bar, Fy_bar).
-__global__ void __launch_bounds__(kSwTX * kSwTY) k_swm_vjp_mid(SwmDev d, const float* __restrict__ y,
-                                                                const float* __restrict__ gbar, float* __restrict__ mid,
-                                                                int bc) {
-    const int b = blockIdx.x * kSwTX + threadIdx.x;
-    const int a = blockIdx.y * kSwTY + threadIdx.y;
-    if (b >= d.Nx || a >= d.Ny) return;
-    const int64_t plane = (int64_t)d.Ny * d.Nx, field = plane * d.nl;
-    const SwmAt F{d, y, plane, field, bc != 0};
-    const int64_t o = (int64_t)a * d.Nx + b;
-    for (int k = 0; k < d.nl; ++k) {
-        const float* gh = gbar + k * plane;
-        const float* gu = gbar + field + k * plane;
-        const float* gv = gbar + 2 * field + k * plane;
-        auto G = [&](const float* g, int j, int i) { return g[(int64_t)j * d.Nx + i]; };
-        float qb = 0.f, vhb = 0.f, uhb = 0.f;
-        if (F.inside(a, b)) {
-            // q(a, b) feeds qU of U(a, b), U(a + 1, b) and qV of V(a, b), V(a, b + 1)
-            qb += 0.5f * (G(gu, a, b) * F.vhU(k, a, b) - G(gv, a, b) * F.uhV(k, a, b));
-            if (F.inside(a + 1, b)) qb += 0.5f * G(gu, a + 1, b) * F.vhU(k, a + 1, b);
-            if (F.inside(a, b + 1)) qb -= 0.5f * G(gv, a, b + 1) * F.uhV(k, a, b + 1);
-            // vh(a, b) feeds vhU of U(a, b), U(a, b - 1), U(a + 1, b), U(a + 1, b - 1)
-            const int uj[4] = {a, a, a + 1, a + 1}, ui[4] = {b, b - 1, b, b - 1};
+__global__ void __launch_bounds__(kVjX * kVjY) k_swm_vjp(SwmDev d, const float* y, const float* gbar,
+                                                         const float* params, float* ybar, double* pacc, int bc) {
+    __shared__ float sh[kVjE], su[kVjE], sv[kVjE];     // stage input
+    __shared__ float gh[kVjE], gu[kVjE], gv[kVjE];     // cotangents of the interior tendencies, else 0
+    __shared__ float sq[kVjE], sx[kVjE], suh[kVjE], svh[kVjE];  // PV, h at X points, u h, v h
+    __shared__ float mq[kVjE], mv[kVjE], mu[kVjE], mp[kVjE];    // cotangents of PV, v h, u h, the potential
+    __shared__ double red[3][kVjX * kVjY / 32];
+    const int tid = threadIdx.x, k = blockIdx.y, tiles_x = (d.Nx + kVjX - 1) / kVjX, tile_y = blockIdx.x / tiles_x;
+    const int i0 = (blockIdx.x - tile_y * tiles_x) * kVjX - 2, j0 = tile_y * kVjY - 2;
+    const int64_t plane = (int64_t)d.Ny * d.Nx, field = plane * d.nl, lo = k * plane;
+    pdl_wait();
+    pdl_launch_dependents();
+    auto inside = [&](int j, int i) { return j >= 1 && j <= d.Ny - 2 && i >= 1 && i <= d.Nx - 2; };
+    for (int e = tid; e < kVjE; e += kVjX * kVjY) {
+        const int r = e / kVjSX, j = j0 + r, i = i0 + e - r * kVjSX;
+        const bool dom = j >= 0 && j < d.Ny && i >= 0 && i < d.Nx, in = inside(j, i);
+        float x[3];
 #pragma unroll
-            for (int t = 0; t < 4; ++t)
-                if (F.inside(uj[t], ui[t])) vhb += 0.25f * G(gu, uj[t], ui[t]) * F.qU(k, uj[t], ui[t]);
-            // uh(a, b) feeds uhV of V(a, b), V(a, b + 1), V(a - 1, b), V(a - 1, b + 1)
-            const int vj[4] = {a, a, a - 1, a - 1}, vi[4] = {b, b + 1, b, b + 1};
-#pragma unroll
-            for (int t = 0; t < 4; ++t)
-                if (F.inside(vj[t], vi[t])) uhb -= 0.25f * G(gv, vj[t], vi[t]) * F.qV(k, vj[t], vi[t]);
+        for (int f = 0; f < 3; ++f) {
+            const int64_t o = dom ? src(d, f, j, i, bc != 0) : -1;
+            x[f] = o >= 0 ? y[f * field + lo + o] : 0.f;
         }
-        // P(a, b): Pc of U(a, b) and V(a, b), Pe of U(a, b - 1), Pn of V(a - 1, b)
-        float Pb = 0.f;
-        if (F.inside(a, b)) Pb += G(gu, a, b) * d.idx + G(gv, a, b) * d.idy;
-        if (F.inside(a, b - 1)) Pb -= G(gu, a, b - 1) * d.idx;
-        if (F.inside(a - 1, b)) Pb -= G(gv, a - 1, b) * d.idy;
-        // the upwind mass flux through the east face of (a, b) (fe of (a, b), fw of (a, b + 1))
-        // and through its north face (gn of (a, b), gs of (a + 1, b))
-        float Fx = 0.f, Fy = 0.f;
-        if (F.inside(a, b)) {
-            Fx -= G(gh, a, b) * d.idx;
-            Fy -= G(gh, a, b) * d.idy;
+        sh[e] = x[0];
+        su[e] = x[1];
+        sv[e] = x[2];
+        const int64_t o = lo + (int64_t)j * d.Nx + i;
+        gh[e] = in ? gbar[o] : 0.f;
+        gu[e] = in ? gbar[field + o] : 0.f;
+        gv[e] = in ? gbar[2 * field + o] : 0.f;
+    }
+    __syncthreads();
+    constexpr int S = kVjSX;
+    for (int e = tid; e < kVjE; e += kVjX * kVjY) {
+        const int r = e / S, c = e - r * S, j = j0 + r, i = i0 + c;
+        float q = 0.f, hx = 1.f, uh = 0.f, vh = 0.f;
+        if (r < kVjSY - 1 && c < S - 1 && inside(j, i)) {
+            const float zeta = (sv[e + 1] - sv[e]) * d.idx - (su[e + S] - su[e]) * d.idy;
+            hx = 0.25f * (sh[e] + sh[e + 1] + sh[e + S] + sh[e + S + 1]);
+            q = (zeta + __ldg(d.fx + j)) / hx;
+            uh = 0.5f * (sh[e] + sh[e + 1]) * su[e];
+            vh = 0.5f * (sh[e] + sh[e + S]) * sv[e];
         }
-        if (F.inside(a, b + 1)) Fx += G(gh, a, b + 1) * d.idx;
-        if (F.inside(a + 1, b)) Fy += G(gh, a + 1, b) * d.idy;
-        float* m = mid + (int64_t)k * 6 * plane + o;
-        m[0] = qb;
-        m[plane] = vhb;
-        m[2 * plane] = uhb;
-        m[3 * plane] = Pb;
-        m[4 * plane] = Fx;
-        m[5 * plane] = Fy;
+        sq[e] = q;
+        sx[e] = hx;
+        suh[e] = uh;
+        svh[e] = vh;
+    }
+    __syncthreads();
+    for (int e = tid; e < kVjE; e += kVjX * kVjY) {
+        const int r = e / S, c = e - r * S, j = j0 + r, i = i0 + c;
+        float qb = 0.f, vhb = 0.f, uhb = 0.f, Pb = 0.f;
+        if (r >= 1 && r < kVjSY - 1 && c >= 1 && c < S - 1) {
+            // P(j, i): Pc of U(j, i) and V(j, i), Pe of U(j, i - 1), Pn of V(j - 1, i)
+            if (inside(j, i)) Pb += gu[e] * d.idx + gv[e] * d.idy;
+            Pb -= gu[e - 1] * d.idx;
+            Pb -= gv[e - S] * d.idy;
+            if (r < kVjSY - 2 && c < S - 2 && inside(j, i)) {
+                auto vhU = [&](int x) { return 0.25f * (svh[x] + svh[x + 1] + svh[x - S] + svh[x - S + 1]); };
+                auto uhV = [&](int x) { return 0.25f * (suh[x] + suh[x - 1] + suh[x + S] + suh[x + S - 1]); };
+                auto qU = [&](int x) { return 0.5f * (sq[x] + sq[x - S]); };
+                auto qV = [&](int x) { return 0.5f * (sq[x] + sq[x - 1]); };
+                // q(j, i) feeds qU of U(j, i), U(j + 1, i) and qV of V(j, i), V(j, i + 1)
+                qb = 0.5f * (gu[e] * vhU(e) - gv[e] * uhV(e)) + 0.5f * gu[e + S] * vhU(e + S) - 0.5f * gv[e + 1] * uhV(e + 1);
+                // vh(j, i) feeds vhU of U(j, i), U(j, i - 1), U(j + 1, i), U(j + 1, i - 1)
+                vhb = 0.25f * gu[e] * qU(e) + 0.25f * gu[e - 1] * qU(e - 1) + 0.25f * gu[e + S] * qU(e + S) +
+                      0.25f * gu[e + S - 1] * qU(e + S - 1);
+                // uh(j, i) feeds uhV of V(j, i), V(j, i + 1), V(j - 1, i), V(j - 1, i + 1)
+                uhb = -0.25f * gv[e] * qV(e) - 0.25f * gv[e + 1] * qV(e + 1) - 0.25f * gv[e - S] * qV(e - S) -
+                      0.25f * gv[e - S + 1] * qV(e - S + 1);
+            }
+        }
+        mq[e] = qb;
+        mv[e] = vhb;
+        mu[e] = uhb;
+        mp[e] = Pb;
+    }
+    __syncthreads();
+    const float nu = params[0], kappa = params[1];
+    const int tx = tid % kVjX, ty = tid / kVjX, e = (ty + 2) * S + tx + 2;
+    const int b = i0 + 2 + tx, a = j0 + 2 + ty;
+    double pnu = 0.0, pkap = 0.0, ptau = 0.0;
+    if (b < d.Nx && a < d.Ny) {
+        const int64_t o = (int64_t)a * d.Nx + b;
+        // the potential's cotangents of the layers below, then this one's
+        float pcum = 0.f;
+        for (int l = d.nl - 1; l > k; --l) {
+            const float *Gu = gbar + field + l * plane + o, *Gv = Gu + field;
+            float Pb = 0.f;
+            if (inside(a, b)) Pb += Gu[0] * d.idx + Gv[0] * d.idy;
+            if (inside(a, b - 1)) Pb -= Gu[-1] * d.idx;
+            if (inside(a - 1, b)) Pb -= Gv[-d.Nx] * d.idy;
+            pcum += Pb;
+        }
+        pcum += mp[e];
+        const float h0 = sh[e], u0 = su[e], v0 = sv[e];
+        const bool in = inside(a, b), east = b + 1 < d.Nx, west = b >= 1, north = a + 1 < d.Ny, south = a >= 1;
+        // the upwind mass flux through the east face of (j, i) (fe of (j, i), fw of (j, i + 1)) and
+        // through its north face (gn of (j, i), gs of (j + 1, i))
+        auto Fx = [&](int x) { return (gh[x + 1] - gh[x]) * d.idx; };
+        auto Fy = [&](int x) { return (gh[x + S] - gh[x]) * d.idy; };
+        float hb = 0.f, ub = 0.f, vb = 0.f;
+        // face (a, b) takes h(a, b) when u(a, b) > 0, face (a, b - 1) takes h(a, b) when
+        // u(a, b - 1) <= 0 (the same in y)
+        if (east) {
+            const float fx = Fx(e);
+            if (u0 > 0.f) hb += fx * u0;
+            ub += fx * (u0 > 0.f ? h0 : sh[e + 1]);
+        }
+        if (west && !(su[e - 1] > 0.f)) hb += Fx(e - 1) * su[e - 1];
+        if (north) {
+            const float fy = Fy(e);
+            if (v0 > 0.f) hb += fy * v0;
+            vb += fy * (v0 > 0.f ? h0 : sh[e + S]);
+        }
+        if (south && !(sv[e - S] > 0.f)) hb += Fy(e - S) * sv[e - S];
+        // PV: q = (zeta + f) / hX at the X points (a, b), (a, b - 1), (a - 1, b), (a - 1, b - 1); mq is
+        // zero where PV is not formed
+        hb -= 0.25f * (mq[e] * sq[e] / sx[e] + mq[e - 1] * sq[e - 1] / sx[e - 1] + mq[e - S] * sq[e - S] / sx[e - S] +
+                       mq[e - S - 1] * sq[e - S - 1] / sx[e - S - 1]);
+        const float z0 = mq[e] / sx[e];
+        ub += (z0 - mq[e - S] / sx[e - S]) * d.idy;
+        vb += (mq[e - 1] / sx[e - 1] - z0) * d.idx;
+        // face mass fluxes of the PV flux: vh(a, b), vh(a - 1, b), uh(a, b), uh(a, b - 1)
+        hb += 0.5f * (mv[e] * v0 + mv[e - S] * sv[e - S]);
+        hb += 0.5f * (mu[e] * u0 + mu[e - 1] * su[e - 1]);
+        vb += mv[e] * 0.5f * (h0 + sh[e + S]);
+        ub += mu[e] * 0.5f * (h0 + sh[e + 1]);
+        // kinetic energy (interior T points): ke(a, b) and ke(a, b + 1) read u(a, b), ke(a, b) and
+        // ke(a + 1, b) read v(a, b)
+        const float pab = in ? mp[e] : 0.f;
+        ub += 0.5f * u0 * (pab + (inside(a, b + 1) ? mp[e + 1] : 0.f));
+        vb += 0.5f * v0 * (pab + (inside(a + 1, b) ? mp[e + S] : 0.f));
+        // Laplacians of the interior outputs (their transpose), and nu's cotangent
+        ub += nu * ((gu[e - 1] + gu[e + 1] - 2.f * gu[e]) * d.idx2 + (gu[e - S] + gu[e + S] - 2.f * gu[e]) * d.idy2);
+        vb += nu * ((gv[e - 1] + gv[e + 1] - 2.f * gv[e]) * d.idx2 + (gv[e - S] + gv[e + S] - 2.f * gv[e]) * d.idy2);
+        if (in) {
+            const float lu = (su[e + 1] - 2.f * u0 + su[e - 1]) * d.idx2 + (su[e + S] - 2.f * u0 + su[e - S]) * d.idy2;
+            const float lv = (sv[e + 1] - 2.f * v0 + sv[e - 1]) * d.idx2 + (sv[e + S] - 2.f * v0 + sv[e - S]) * d.idy2;
+            pnu = (double)(gu[e] * lu + gv[e] * lv);
+        }
+        // drag (bottom layer, every cell) and wind (top layer, every cell)
+        const float guo = gbar[field + lo + o], gvo = gbar[2 * field + lo + o];
+        if (k == d.nl - 1) {
+            ub -= kappa * guo;
+            vb -= kappa * gvo;
+            pkap = -(double)(guo * u0 + gvo * v0);
+        }
+        if (k == 0) ptau = (double)(guo * __ldg(d.wx + a) * d.invH0);
+        hb += __ldg(d.gp + k) * pcum;
+        ybar[lo + o] = hb;
+        ybar[field + lo + o] = ub;
+        ybar[2 * field + lo + o] = vb;
+    }
+    // parameter cotangents: one double atomic a CTA
+    for (int m = 16; m > 0; m >>= 1) {
+        pnu += __shfl_down_sync(0xffffffffu, pnu, m);
+        pkap += __shfl_down_sync(0xffffffffu, pkap, m);
+        ptau += __shfl_down_sync(0xffffffffu, ptau, m);
+    }
+    if ((tid & 31) == 0) {
+        red[0][tid >> 5] = pnu;
+        red[1][tid >> 5] = pkap;
+        red[2][tid >> 5] = ptau;
+    }
+    __syncthreads();
+    if (tid < 3) {
+        double v = 0.0;
+        for (int w = 0; w < kVjX * kVjY / 32; ++w) v += red[tid][w];
+        if (tid == 0 || (tid == 1 && k == d.nl - 1) || (tid == 2 && k == 0)) atomicAdd(pacc + tid, v);
     }
 }
 
-// The stage-input cotangent at (a, b) of every layer and the parameter cotangents
-// (accumulated in pacc[0..2] as doubles: nu, kappa, tau0).
-__global__ void __launch_bounds__(kSwTX * kSwTY) k_swm_vjp_in(SwmDev d, const float* __restrict__ y,
-                                                               const float* __restrict__ gbar,
-                                                               const float* __restrict__ mid,
-                                                               const float* __restrict__ params, float* ybar,
-                                                               double* pacc, int bc) {
-    const int b = blockIdx.x * kSwTX + threadIdx.x;
-    const int a = blockIdx.y * kSwTY + threadIdx.y;
-    const bool mine = b < d.Nx && a < d.Ny;
-    const int64_t plane = (int64_t)d.Ny * d.Nx, field = plane * d.nl;
-    const float nu = params[0], kappa = params[1];
-    float pnu = 0.f, pkap = 0.f, ptau = 0.f;
-    if (mine) {
-        const SwmAt F{d, y, plane, field, bc != 0};
-        const int64_t o = (int64_t)a * d.Nx + b;
-        auto M = [&](int k, int c, int j, int i) { return mid[((int64_t)k * 6 + c) * plane + (int64_t)j * d.Nx + i]; };
-        float pcum = 0.f;  // sum over the layers k >= l of P_bar_k(a, b)
-        for (int k = d.nl - 1; k >= 0; --k) {
-            const float* gu = gbar + field + k * plane;
-            const float* gv = gbar + 2 * field + k * plane;
-            auto G = [&](const float* g, int j, int i) { return F.inside(j, i) ? g[(int64_t)j * d.Nx + i] : 0.f; };
-            const float h0 = F.H(k, a, b), u0 = F.U(k, a, b), v0 = F.V(k, a, b);
-            const bool east = b + 1 < d.Nx, west = b >= 1, north = a + 1 < d.Ny, south = a >= 1;
-            pcum += M(k, 3, a, b);
-            float hb = 0.f;  // the pressure sum's share g'_k sum_{k' >= k} P_bar_k' is added last
-            // upwind mass fluxes: face (a, b) takes h(a, b) when u(a, b) > 0, face (a, b - 1) takes
-            // h(a, b) when u(a, b - 1) <= 0 (the same in y)
-            float ub = 0.f, vb = 0.f;
-            if (east) {
-                const float fx = M(k, 4, a, b);
-                if (u0 > 0.f) hb += fx * u0;
-                ub += fx * (u0 > 0.f ? h0 : F.H(k, a, b + 1));
-            }
-            if (west) {
-                const float uw = F.U(k, a, b - 1);
-                if (!(uw > 0.f)) hb += M(k, 4, a, b - 1) * uw;
-            }
-            if (north) {
-                const float fy = M(k, 5, a, b);
-                if (v0 > 0.f) hb += fy * v0;
-                vb += fy * (v0 > 0.f ? h0 : F.H(k, a + 1, b));
-            }
-            if (south) {
-                const float vs = F.V(k, a - 1, b);
-                if (!(vs > 0.f)) hb += M(k, 5, a - 1, b) * vs;
-            }
-            // PV: q = (zeta + f) / hX at the X points (a, b), (a, b - 1), (a - 1, b), (a - 1, b - 1)
-            auto zb = [&](int j, int i) {  // zeta_bar = q_bar / hX
-                return F.inside(j, i) ? M(k, 0, j, i) / F.hX(k, j, i) : 0.f;
-            };
-            const int xj[4] = {a, a, a - 1, a - 1}, xi[4] = {b, b - 1, b, b - 1};
-#pragma unroll
-            for (int t = 0; t < 4; ++t)
-                if (F.inside(xj[t], xi[t])) hb -= 0.25f * M(k, 0, xj[t], xi[t]) * F.qX(k, xj[t], xi[t]) / F.hX(k, xj[t], xi[t]);
-            ub += (zb(a, b) - (south ? zb(a - 1, b) : 0.f)) * d.idy;
-            vb += ((west ? zb(a, b - 1) : 0.f) - zb(a, b)) * d.idx;
-            // face mass fluxes of the PV flux: vh(a, b), vh(a - 1, b), uh(a, b), uh(a, b - 1)
-            hb += 0.5f * (M(k, 1, a, b) * v0 + (south ? M(k, 1, a - 1, b) * F.V(k, a - 1, b) : 0.f));
-            hb += 0.5f * (M(k, 2, a, b) * u0 + (west ? M(k, 2, a, b - 1) * F.U(k, a, b - 1) : 0.f));
-            if (north) vb += M(k, 1, a, b) * 0.5f * (h0 + F.H(k, a + 1, b));
-            if (east) ub += M(k, 2, a, b) * 0.5f * (h0 + F.H(k, a, b + 1));
-            // kinetic energy (interior T points): ke(a, b) and ke(a, b + 1) read u(a, b),
-            // ke(a, b) and ke(a + 1, b) read v(a, b)
-            const float pab = F.inside(a, b) ? M(k, 3, a, b) : 0.f;
-            ub += 0.5f * u0 * (pab + (east && F.inside(a, b + 1) ? M(k, 3, a, b + 1) : 0.f));
-            vb += 0.5f * v0 * (pab + (north && F.inside(a + 1, b) ? M(k, 3, a + 1, b) : 0.f));
-            // Laplacians of the interior outputs (their transpose), and nu's cotangent
-            const float gc = G(gu, a, b), gvc = G(gv, a, b);
-            ub += nu * (((west ? G(gu, a, b - 1) : 0.f) + (east ? G(gu, a, b + 1) : 0.f) - 2.f * gc) * d.idx2 +
-                        ((south ? G(gu, a - 1, b) : 0.f) + (north ? G(gu, a + 1, b) : 0.f) - 2.f * gc) * d.idy2);
-            vb += nu * (((west ? G(gv, a, b - 1) : 0.f) + (east ? G(gv, a, b + 1) : 0.f) - 2.f * gvc) * d.idx2 +
-                        ((south ? G(gv, a - 1, b) : 0.f) + (north ? G(gv, a + 1, b) : 0.f) - 2.f * gvc) * d.idy2);
-            if (F.inside(a, b)) {
-                const float lu = (F.U(k, a, b + 1) - 2.f * u0 + F.U(k, a, b - 1)) * d.idx2 +
-                                 (F.U(k, a + 1, b) - 2.f * u0 + F.U(k, a - 1, b)) * d.idy2;
-                const float lv = (F.V(k, a, b + 1) - 2.f * v0 + F.V(k, a, b - 1)) * d.idx2 +
-                                 (F.V(k, a + 1, b) - 2.f * v0 + F.V(k, a - 1, b)) * d.idy2;
-                pnu += gc * lu + gvc * lv;
-            }
-            // drag (bottom layer, every cell) and wind (top layer, every cell)
-            const float guo = gu[o], gvo = gv[o];
-            if (k == d.nl - 1) {
-                ub -= kappa * guo;
-                vb -= kappa * gvo;
-                pkap -= guo * u0 + gvo * v0;
-            }
-            if (k == 0) ptau += guo * __ldg(d.wx + a) * d.invH0;
-            hb += __ldg(d.gp + k) * pcum;
-            ybar[k * plane + o] = hb;
-            ybar[field + k * plane + o] = ub;
-            ybar[2 * field + k * plane + o] = vb;
+// The other rows (columns) whose values field f takes from row (column) x of n points under the
+// boundary rules, or -1; walls: `fixed` fields do not copy along this axis.
+__device__ __forceinline__ int copied_by(const SwmDev& d, int x, int n, bool fixed) {
+    if (d.bc == QG_SWM_PERIODIC) return x == 1 ? n - 1 : (x == n - 2 ? 0 : -1);
+    if (fixed) return -1;
+    return x == 1 ? 0 : (x == n - 2 ? n - 1 : -1);
+}
+
+struct Scatter {
+    float* k[kMaxButcher];  // cotangents of the earlier stage derivatives
+    float c[kMaxButcher];
+    int n;
+};
+
+// t = B^T x (with bc: the transpose of the boundary rules), then y += t and k_m += c_m t; cells that
+// the rules overwrite have t = 0.
+__global__ void __launch_bounds__(256) k_swm_scatter(SwmDev d, float* y, const float* x, Scatter sc, int bc) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int64_t plane = (int64_t)d.Ny * d.Nx;
+    const int fk = blockIdx.y, f = fk / d.nl;  // field and layer
+    for (int64_t c = blockIdx.x * (int64_t)256 + threadIdx.x; c < plane; c += (int64_t)gridDim.x * 256) {
+        const int64_t o = fk * plane + c;
+        float t = x[o];
+        if (bc) {
+            const int j = (int)(c / d.Nx), i = (int)(c - (int64_t)j * d.Nx);
+            int jj = j, ii = i;
+            if (!src_cell(d, f, jj, ii) || jj != j || ii != i) continue;
+            const int jr = copied_by(d, j, d.Ny, f == 2), ir = copied_by(d, i, d.Nx, f == 1);
+            const float* p = x + fk * plane;
+            if (jr >= 0) t += p[(int64_t)jr * d.Nx + i];
+            if (ir >= 0) t += p[(int64_t)j * d.Nx + ir];
+            if (jr >= 0 && ir >= 0) t += p[(int64_t)jr * d.Nx + ir];
         }
+        y[o] += t;
+#pragma unroll
+        for (int m = 0; m < kMaxButcher; ++m)
+            if (m < sc.n) sc.k[m][o] = fmaf(sc.c[m], t, sc.k[m][o]);
     }
-    // parameter cotangents: warp sums, one double atomic per warp
-    for (int sh = 16; sh > 0; sh >>= 1) {
-        pnu += __shfl_down_sync(0xffffffffu, pnu, sh);
-        pkap += __shfl_down_sync(0xffffffffu, pkap, sh);
-        ptau += __shfl_down_sync(0xffffffffu, ptau, sh);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(pacc + 0, (double)pnu);
-        atomicAdd(pacc + 1, (double)pkap);
-        atomicAdd(pacc + 2, (double)ptau);
+}
+
+// k_m = c_m x over n floats
+__global__ void __launch_bounds__(256) k_swm_fanout(const float* x, Scatter sc, int64_t n) {
+    pdl_wait();
+    pdl_launch_dependents();
+    for (int64_t t = blockIdx.x * (int64_t)256 + threadIdx.x; t < n; t += (int64_t)gridDim.x * 256) {
+        const float v = x[t];
+#pragma unroll
+        for (int m = 0; m < kMaxButcher; ++m)
+            if (m < sc.n) sc.k[m][t] = sc.c[m] * v;
     }
 }
 
@@ -805,11 +837,9 @@ __global__ void k_swm_bc_vjp(SwmDev d, float* ybar) {
     }
 }
 
-// y += alpha x, and y = alpha x, over n floats
-__global__ void k_swm_axpy(float* y, const float* __restrict__ x, float alpha, int64_t n, int overwrite) {
-    const int64_t nth = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += nth)
-        y[t] = overwrite ? alpha * x[t] : fmaf(alpha, x[t], y[t]);
+// A kernel and not a memset: a launch that may start early follows it in captured graphs.
+__global__ void k_swm_pzero(double* pacc) {
+    if (threadIdx.x < 4) pacc[threadIdx.x] = 0.0;
 }
 
 __global__ void k_swm_pbar(const double* pacc, float* pbar, int accumulate) {
@@ -864,7 +894,6 @@ struct qg_swm_plan {
     float* params = nullptr;  // plan-owned copy of the params (graph-stable)
     float* proj = nullptr;    // projected stage input of qg_reparam_step
     void* stats_acc = nullptr;  // qg_swm_state_stats accumulators
-    float* mid = nullptr;       // the VJP's mid-point cotangents (6 planes per layer)
     double* pacc = nullptr;     // the VJP's parameter cotangent sums
     // qg_swm_step_vjp replayed as a captured graph while its pointers, dt and scheme repeat
     cudaGraphExec_t vjp_exec = nullptr;
@@ -976,7 +1005,6 @@ extern "C" int qg_swm_create(const qg_swm_desc* desc, qg_swm_plan** out) {
     if (!e) e = cudaMemset(p->params, 0, 4 * sizeof(float));
     if (!e) e = cudaMalloc(&p->proj, p->n * sizeof(float));
     if (!e) e = cudaMalloc(&p->stats_acc, 64);
-    if (!e) e = cudaMalloc(&p->mid, (size_t)6 * d.nl * d.Ny * d.Nx * sizeof(float));
     if (!e) e = cudaMalloc(&p->pacc, 4 * sizeof(double));
     if (!e) e = cudaMalloc(&p->flags, 16);
     if (!e) e = cudaMemset(p->flags, 0, 16);
@@ -1004,7 +1032,7 @@ extern "C" void qg_swm_destroy(qg_swm_plan* p) {
         }
     if (p->cap) cudaStreamDestroy(p->cap);
     for (void* a : {(void*)p->consts, (void*)p->stage, (void*)p->K, (void*)p->params, (void*)p->proj,
-                    p->stats_acc, (void*)p->mid, (void*)p->pacc, (void*)p->flags})
+                    p->stats_acc, (void*)p->pacc, (void*)p->flags})
         if (a) cudaFree(a);
     delete p;
 }
@@ -1012,27 +1040,52 @@ extern "C" void qg_swm_destroy(qg_swm_plan* p) {
 extern "C" int64_t qg_swm_state_size(const qg_swm_plan* p) { return p ? p->n : -1; }
 
 namespace {
+// A launch that may start while the kernel before it finishes (programmatic dependent launch; not
+// while profiling, where events separate the launches).  Only for kernels that wait for it.
+template <class... KArgs, class... Args>
+cudaError_t swm_launch(const qg_swm_plan* p, void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s,
+                       Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = p->profiling ? 0 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
 // One fused stage launch (k_swm_stage) on stream s.
 template <int NS>
-void launch_ns(const qg_swm_plan* p, const StageArgs& a, cudaStream_t s) {
-    if (a.last)
-        k_swm_stage<NS, true><<<swm_grid(p->d), dim3(kSwTX, kSwTY), 0, s>>>(p->d, a);
-    else
-        k_swm_stage<NS, false><<<swm_grid(p->d), dim3(kSwTX, kSwTY), 0, s>>>(p->d, a);
+cudaError_t launch_ns(const qg_swm_plan* p, const StageArgs& a, cudaStream_t s) {
+    const dim3 g = swm_grid(p->d), b(kSwTX, kSwTY);
+    if (a.ysave) {
+        if (a.last)
+            k_swm_stage<NS, true, true><<<g, b, 0, s>>>(p->d, a);
+        else
+            k_swm_stage<NS, false, true><<<g, b, 0, s>>>(p->d, a);
+    } else {
+        if (a.last)
+            k_swm_stage<NS, true, false><<<g, b, 0, s>>>(p->d, a);
+        else
+            k_swm_stage<NS, false, false><<<g, b, 0, s>>>(p->d, a);
+    }
+    return cudaGetLastError();
 }
 
 cudaError_t launch_stage(const qg_swm_plan* p, const StageArgs& a, cudaStream_t s) {
     static_assert(kMaxButcher == 6, "one instantiation per stage count");
     switch (a.ns) {
-        case 0: launch_ns<0>(p, a, s); break;
-        case 1: launch_ns<1>(p, a, s); break;
-        case 2: launch_ns<2>(p, a, s); break;
-        case 3: launch_ns<3>(p, a, s); break;
-        case 4: launch_ns<4>(p, a, s); break;
-        case 5: launch_ns<5>(p, a, s); break;
+        case 0: return launch_ns<0>(p, a, s);
+        case 1: return launch_ns<1>(p, a, s);
+        case 2: return launch_ns<2>(p, a, s);
+        case 3: return launch_ns<3>(p, a, s);
+        case 4: return launch_ns<4>(p, a, s);
+        case 5: return launch_ns<5>(p, a, s);
         default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 
 StageArgs stage_args(const qg_swm_plan* p, const float* y, float* out, const float* params, int bc) {
@@ -1396,15 +1449,38 @@ extern "C" int qg_reparam_step(qg_swm_plan* p, qg_plan* qp, float* state, const 
 }
 
 namespace {
-// ybar = (the transpose of vector_field's Jacobian at y, with the boundary rules on read when bc)
-// applied to gbar; the parameter cotangents added to p->pacc.
+// ybar = (the transpose of vector_field's Jacobian at y, with the boundary rules on read when bc,
+// up to the rules' own transpose) applied to gbar; the parameter cotangents added to p->pacc.
 cudaError_t swm_vjp(qg_swm_plan* p, const float* y, const float* params, const float* gbar, float* ybar, int bc,
                     cudaStream_t s) {
-    const dim3 g = swm_grid(p->d), b(kSwTX, kSwTY);
-    k_swm_vjp_mid<<<g, b, 0, s>>>(p->d, y, gbar, p->mid, bc);
-    k_swm_vjp_in<<<g, b, 0, s>>>(p->d, y, gbar, p->mid, params, ybar, p->pacc, bc);
-    if (bc) k_swm_bc_vjp<<<g, b, 0, s>>>(p->d, ybar);
-    return cudaGetLastError();
+    const SwmDev& d = p->d;
+    return swm_launch(p, k_swm_vjp, dim3((d.Nx + kVjX - 1) / kVjX * ((d.Ny + kVjY - 1) / kVjY), d.nl), dim3(kVjX * kVjY), s,
+                      d, y, gbar, params, ybar, p->pacc, bc);
+}
+
+// y_bar += t and kb_m += dt a[m] t (m < n, a[m] != 0) with t = x, or the rules' transpose of x
+cudaError_t swm_scatter(qg_swm_plan* p, float* y_bar, const float* x, float* kb, const double* a, int n, double dt,
+                        int bc, cudaStream_t s) {
+    Scatter sc{};
+    for (int m = 0; m < n; ++m)
+        if (a[m] != 0.0) {
+            sc.k[sc.n] = kb + m * p->n;
+            sc.c[sc.n++] = (float)(dt * a[m]);
+        }
+    const int64_t plane = (int64_t)p->d.Ny * p->d.Nx;
+    return swm_launch(p, k_swm_scatter, dim3((unsigned)std::min<int64_t>(2048, (plane + 255) / 256), 3 * p->d.nl),
+                      dim3(256), s, p->d, y_bar, x, sc, bc);
+}
+
+// kb_m = dt b[m] y_bar for every stage
+cudaError_t swm_fanout(qg_swm_plan* p, const float* y_bar, float* kb, const Tableau* tb, double dt, cudaStream_t s) {
+    Scatter sc{};
+    for (sc.n = 0; sc.n < tb->n; ++sc.n) {
+        sc.k[sc.n] = kb + sc.n * p->n;
+        sc.c[sc.n] = (float)(dt * tb->b[sc.n]);
+    }
+    return swm_launch(p, k_swm_fanout, dim3((unsigned)std::min<int64_t>(4096, (p->n + 255) / 256)), dim3(256), s, y_bar,
+                      sc, p->n);
 }
 
 const Tableau* swm_scheme(int scheme) { return swm_tableau(scheme); }
@@ -1415,8 +1491,13 @@ extern "C" int qg_swm_rhs_vjp(qg_swm_plan* p, const float* state, const float* p
     if (!p || !state || !params || !tend_bar || !state_bar || !params_bar) return QG_ERR_NULL;
     if (flags & ~QG_RHS_APPLY_BC) return QG_ERR_ARG;
     cudaStream_t s = (cudaStream_t)stream;
-    cudaError_t e = cudaMemsetAsync(p->pacc, 0, 4 * sizeof(double), s);
+    k_swm_pzero<<<1, 32, 0, s>>>(p->pacc);
+    cudaError_t e = cudaGetLastError();
     if (!e) e = swm_vjp(p, state, params, tend_bar, state_bar, flags & QG_RHS_APPLY_BC, s);
+    if (!e && (flags & QG_RHS_APPLY_BC)) {
+        k_swm_bc_vjp<<<swm_grid(p->d), dim3(kSwTX, kSwTY), 0, s>>>(p->d, state_bar);
+        e = cudaGetLastError();
+    }
     if (!e) {
         k_swm_pbar<<<1, 32, 0, s>>>(p->pacc, params_bar, 0);
         e = cudaGetLastError();
@@ -1437,50 +1518,72 @@ extern "C" int64_t qg_swm_step_vjp_workspace(const qg_swm_plan* p, int scheme) {
 }
 
 namespace {
+// The stages of one step from y: their derivatives into K, the stage inputs 1 .. n - 1 into Y (n
+// floats each, their boundary values as the rules read them; null: not kept) and the next state
+// into y_next (null: only what the stage inputs need).  The arithmetic is qg_swm_step's.
+cudaError_t swm_stages(qg_swm_plan* p, const float* y, const float* params, double dt, const Tableau* tb, float* K,
+                       float* Y, float* y_next, cudaStream_t s) {
+    for (int st = 0; st < tb->n; ++st) {
+        const bool last = st == tb->n - 1;
+        if (last && !y_next) {
+            if (!Y || st == 0) return cudaSuccess;
+            Combine c{};
+            for (int m = 0; m < st; ++m) c.c[m] = (float)(dt * tb->a[st][m]);
+            const int grid = (int)std::min<int64_t>(4096, (p->n + 255) / 256);
+            k_swm_combine<<<grid, 256, 0, s>>>(Y + (st - 1) * p->n, y, K, p->n, st, c);
+            return cudaGetLastError();
+        }
+        StageArgs a = stage_args(p, y, last ? y_next : K + st * p->n, params, 1);
+        a.K = K;
+        a.ns = st;
+        a.last = last;
+        a.ysave = Y && st > 0 ? Y + (st - 1) * p->n : nullptr;
+        for (int m = 0; m < st; ++m) a.a[m] = (float)(dt * tb->a[st][m]);
+        for (int m = 0; last && m < tb->n; ++m) a.b[m] = (float)(dt * tb->b[m]);
+        const cudaError_t e = launch_stage(p, a, s);
+        if (e) return e;
+    }
+    return cudaSuccess;
+}
+
+// The reverse sweep of one step over its stage inputs (y, Y): Kbar_s = dt b_s ybar, then the
+// stages in reverse, Ybar = F_vjp(Y_s; Kbar_s), y0_bar += Ybar, Kbar_m += dt a_sm Ybar; Kb holds n
+// derivatives' cotangents, Yb one state.
+cudaError_t swm_reverse(qg_swm_plan* p, const float* y, const float* Y, const float* params, double dt,
+                        const Tableau* tb, float* y_bar, float* Kb, float* Yb, cudaStream_t s) {
+    cudaError_t e = swm_fanout(p, y_bar, Kb, tb, dt, s);
+    for (int st = tb->n - 1; st >= 0 && !e; --st) {
+        e = swm_vjp(p, st == 0 ? y : Y + (st - 1) * p->n, params, Kb + st * p->n, Yb, 1, s);
+        if (!e) e = swm_scatter(p, y_bar, Yb, Kb, tb->a[st], st, dt, 1, s);
+    }
+    return e;
+}
+
 // The launches of one step's adjoint on stream s (see qg_swm_step_vjp).
 cudaError_t swm_step_vjp_body(qg_swm_plan* p, const float* y0, const float* params, double dt, const Tableau* tb,
-                              float* y_bar, float* params_bar, float* work, cudaStream_t s, bool own_pacc = true) {
+                              float* y_bar, float* params_bar, float* work, cudaStream_t s) {
     const int ns = tb->n;
     const int64_t n = p->n;
-    const int cgrid = (int)std::min<int64_t>(4096, (n + 255) / 256);
-    // work: stage inputs Y_1 .. Y_{ns-1}, stage derivatives K_0 .. K_{ns-2} (contiguous), their
-    // cotangents Kbar_0 .. Kbar_{ns-1}, one stage-input cotangent
-    const float* Y[kMaxButcher];
-    Y[0] = y0;
-    for (int i = 1; i < ns; ++i) Y[i] = work + (int64_t)(i - 1) * n;
-    float* K = work + (int64_t)(ns - 1) * n;
-    float* Kb = work + (int64_t)(2 * ns - 2) * n;
-    float* Yb = work + (int64_t)(3 * ns - 2) * n;
-    cudaError_t e = cudaSuccess;
-    // the step's stage inputs again: Y_s = y0 + dt sum_m a_sm K_m, K_m = F(B(Y_m))
-    for (int st = 0; st + 1 < ns && !e; ++st) {
-        e = launch_stage(p, stage_args(p, Y[st], K + st * n, params, 1), s);
-        if (e) break;
-        Combine c{};
-        for (int m = 0; m <= st; ++m) c.c[m] = (float)(dt * tb->a[st + 1][m]);
-        k_swm_combine<<<cgrid, 256, 0, s>>>(const_cast<float*>(Y[st + 1]), y0, K, n, st + 1, c);
+    // work: stage inputs Y_1 .. Y_{ns-1}, stage derivatives K_0 .. K_{ns-2}, their cotangents
+    // Kbar_0 .. Kbar_{ns-1}, one stage-input cotangent
+    float *Y = work, *K = Y + (ns - 1) * n, *Kb = K + (ns - 1) * n, *Yb = Kb + ns * n;
+    cudaError_t e = swm_stages(p, y0, params, dt, tb, K, Y, nullptr, s);
+    if (!e) {
+        k_swm_pzero<<<1, 32, 0, s>>>(p->pacc);
         e = cudaGetLastError();
     }
-    // Kbar_s = dt b_s ybar, then the stages in reverse: Ybar = F_vjp(Y_s; Kbar_s),
-    // y0_bar += Ybar, Kbar_m += dt a_sm Ybar
-    for (int st = 0; st < ns && !e; ++st) {
-        k_swm_axpy<<<cgrid, 256, 0, s>>>(Kb + st * n, y_bar, (float)(dt * tb->b[st]), n, 1);
-        e = cudaGetLastError();
-    }
-    if (!e && own_pacc) e = cudaMemsetAsync(p->pacc, 0, 4 * sizeof(double), s);
-    for (int st = ns - 1; st >= 0 && !e; --st) {
-        e = swm_vjp(p, Y[st], params, Kb + st * n, Yb, 1, s);
-        if (e) break;
-        k_swm_axpy<<<cgrid, 256, 0, s>>>(y_bar, Yb, 1.f, n, 0);
-        for (int m = 0; m < st; ++m)
-            if (tb->a[st][m] != 0.0) k_swm_axpy<<<cgrid, 256, 0, s>>>(Kb + m * n, Yb, (float)(dt * tb->a[st][m]), n, 0);
-        e = cudaGetLastError();
-    }
-    if (!e && own_pacc) {
+    if (!e) e = swm_reverse(p, y0, Y, params, dt, tb, y_bar, Kb, Yb, s);
+    if (!e) {
         k_swm_pbar<<<1, 32, 0, s>>>(p->pacc, params_bar, 0);
         e = cudaGetLastError();
     }
     return e;
+}
+
+// Whether a segment of k steps keeps every step's stage inputs (up to 1 GiB of them): each step's
+// stages then run once, where the reverse sweep otherwise runs them again.
+bool swm_keeps_inputs(const qg_swm_plan* p, const Tableau* tb, int k) {
+    return (int64_t)(tb->n - 1) * k * p->n * (int64_t)sizeof(float) <= (int64_t)1 << 30;
 }
 
 // The adjoint of k steps from y_start on stream s: the k - 1 later states recomputed into
@@ -1489,19 +1592,24 @@ cudaError_t swm_step_vjp_body(qg_swm_plan* p, const float* y0, const float* para
 cudaError_t swm_segment_vjp_body(qg_swm_plan* p, const float* y_start, const float* params, double dt,
                                  const Tableau* tb, int k, float* y_bar, float* params_bar, float* work,
                                  cudaStream_t s) {
+    const int ns = tb->n;
     const int64_t n = p->n;
-    float* states = work;                        // y_1 .. y_{k-1}
-    float* vwork = work + (int64_t)(k - 1) * n;  // one step's adjoint workspace
+    const bool keep = swm_keeps_inputs(p, tb, k);
+    // work: the states y_1 .. y_{k-1}, stage derivatives, their cotangents, one stage-input
+    // cotangent, the stage inputs of every step or of one
+    float *states = work, *K = states + (k - 1) * n, *Kb = K + (ns - 1) * n, *Yb = Kb + ns * n, *Y = Yb + n;
+    auto state = [&](int i) { return i == 0 ? y_start : states + (i - 1) * n; };
+    auto inputs = [&](int i) { return keep ? Y + (int64_t)i * (ns - 1) * n : Y; };
     cudaError_t e = cudaSuccess;
-    for (int i = 1; i < k && !e; ++i) {
-        float* y = states + (int64_t)(i - 1) * n;
-        e = cudaMemcpyAsync(y, i == 1 ? y_start : y - n, n * sizeof(float), cudaMemcpyDeviceToDevice, s);
-        if (!e) e = swm_steps(p, y, tb, dt, 1, s);
+    for (int i = 0; i + 1 < k && !e; ++i)
+        e = swm_stages(p, state(i), params, dt, tb, K, keep ? inputs(i) : nullptr, states + i * n, s);
+    if (!e) {
+        k_swm_pzero<<<1, 32, 0, s>>>(p->pacc);
+        e = cudaGetLastError();
     }
-    if (!e) e = cudaMemsetAsync(p->pacc, 0, 4 * sizeof(double), s);
     for (int i = k - 1; i >= 0 && !e; --i) {
-        const float* y = i == 0 ? y_start : states + (int64_t)(i - 1) * n;
-        e = swm_step_vjp_body(p, y, params, dt, tb, y_bar, params_bar, vwork, s, false);
+        if (!keep || i == k - 1) e = swm_stages(p, state(i), params, dt, tb, K, inputs(i), nullptr, s);
+        if (!e) e = swm_reverse(p, state(i), inputs(i), params, dt, tb, y_bar, Kb, Yb, s);
     }
     if (!e) {
         k_swm_pbar<<<1, 32, 0, s>>>(p->pacc, params_bar, 0);
@@ -1552,7 +1660,7 @@ extern "C" int qg_swm_step_vjp(qg_swm_plan* p, const float* y0, const float* par
 extern "C" int64_t qg_swm_segment_vjp_workspace(const qg_swm_plan* p, int scheme, int k) {
     const Tableau* tb = swm_scheme(scheme);
     if (!p || !tb || k < 1) return -1;
-    return (int64_t)(k - 1 + 3 * tb->n - 1) * p->n;
+    return (int64_t)(k - 1 + 2 * tb->n + (tb->n - 1) * (swm_keeps_inputs(p, tb, k) ? k : 1)) * p->n;
 }
 
 extern "C" int qg_swm_segment_vjp(qg_swm_plan* p, const float* y_start, const float* params, double dt, int k,
@@ -1675,20 +1783,14 @@ extern "C" int qg_reparam_step_vjp(qg_swm_plan* p, qg_plan* qp, const float* y0,
         if (cudaGetLastError() != cudaSuccess) return QG_ERR_CUDA;
     }
     if (r != QG_OK) return r;
-    for (int st = 0; st < ns && !e; ++st) {
-        k_swm_axpy<<<cgrid, 256, 0, s>>>(Kb + st * n, y_bar, (float)(dt * tb->b[st]), n, 1);
-        e = cudaGetLastError();
-    }
+    e = swm_fanout(p, y_bar, Kb, tb, dt, s);
     if (!e) e = cudaMemsetAsync(p->pacc, 0, 4 * sizeof(double), s);
     for (int st = ns - 1; st >= 0 && !e; --st) {
         e = swm_vjp(p, Z + st * n, params, Kb + st * n, Zb, 0, s);
         if (e) break;
         r = reparam_bc_project_vjp(p, qp, Zb, T, s);
         if (r != QG_OK) return r;
-        k_swm_axpy<<<cgrid, 256, 0, s>>>(y_bar, T, 1.f, n, 0);
-        for (int m = 0; m < st; ++m)
-            if (tb->a[st][m] != 0.0) k_swm_axpy<<<cgrid, 256, 0, s>>>(Kb + m * n, T, (float)(dt * tb->a[st][m]), n, 0);
-        e = cudaGetLastError();
+        e = swm_scatter(p, y_bar, T, Kb, tb->a[st], st, dt, 0, s);
     }
     if (!e) {
         k_swm_pbar<<<1, 32, 0, s>>>(p->pacc, params_bar, 0);
