@@ -293,6 +293,11 @@ int qg_plan_engine(const qg_plan* plan, int* cluster_ctas, float* ms, int n);
    reference counterpart. */
 int qg_plan_row_engine(const qg_plan* plan, int* on, float* ms);
 
+/* dst (device) = n host floats, in stream order without waiting for the stream: they travel as
+   kernel arguments and may change once the call returns.  For parameter vectors (a launch per
+   1024 values).  No reference counterpart. */
+int qg_write(float* dst, const float* values, int64_t n, void* stream);
+
 /* ---------------------------------------------------------------------------------------
    Multilayer shallow-water right-hand side: MultilayerShallowWater2D
    (somax/_src/models/swm/multilayer.py:150-200 vector_field, :202-219 apply_boundary_conditions,

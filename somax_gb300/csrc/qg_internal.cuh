@@ -230,6 +230,7 @@ cudaError_t launch_lsweep_group(const StencilArgs& a, const SweepItem* items, in
 
 // launchers (return cudaError_t of the launch)
 cudaError_t launch_prep(const PrepArgs& a, int ntiles, cudaStream_t s, bool pdl);
+cudaError_t launch_write(float* dst, const float* values, int64_t n, cudaStream_t s);
 cudaError_t launch_unpack(const MemberDev* members, const StencilTile* tiles, int ntiles, int large,
                           const float* src, float* q, cudaStream_t s, bool pdl);
 cudaError_t launch_mode_to_layer(const MemberDev* members, const StencilTile* tiles, int ntiles, int large,

@@ -1473,6 +1473,12 @@ cudaError_t rhs_core(qg_plan* p, const float* q, float* dq, const float* params,
 }
 }  // namespace
 
+int qg_write(float* dst, const float* values, int64_t n, void* stream) {
+    if (n < 0) return QG_ERR_ARG;
+    if (n > 0 && (!dst || !values)) return QG_ERR_NULL;
+    return cuda_err(launch_write(dst, values, n, (cudaStream_t)stream));
+}
+
 int qg_rhs(qg_plan* p, const float* q, float* dq, const float* params, int flags, void* stream) {
     if (!p || !q || !dq || !params) return QG_ERR_NULL;
     if (flags & ~QG_RHS_APPLY_BC) return QG_ERR_ARG;

@@ -9,6 +9,7 @@
 // anything a predecessor kernel writes only after it.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cstring>
 
 #include "qg_stencil_tile.cuh"
@@ -552,6 +553,34 @@ cudaError_t launch_prep(const PrepArgs& a, int ntiles, cudaStream_t s, bool pdl)
 
 cudaError_t launch_rk_combine(const RkCombineArgs& a, int ntiles, cudaStream_t s, bool pdl) {
     return launch_k(k_rk_combine, ntiles, NTHREADS, 0, s, pdl, a);
+}
+
+namespace {
+// Host values as kernel arguments.  Bound: the launch.  A pageable copy of a parameter vector takes
+// 19 us of the host's time and waits for all the work ahead of it in the stream, which left the
+// device idle between the calls of a user's loop.
+template <int N>
+struct Values {
+    float v[N];
+};
+template <int N>
+__global__ void k_write(float* __restrict__ dst, Values<N> a, int n) {
+    if ((int)threadIdx.x < n) dst[threadIdx.x] = a.v[threadIdx.x];
+}
+template <int N>
+cudaError_t write_n(float* dst, const float* values, int n, cudaStream_t s) {
+    Values<N> a;
+    std::copy(values, values + n, a.v);
+    k_write<N><<<1, N, 0, s>>>(dst, a, n);
+    return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t launch_write(float* dst, const float* values, int64_t n, cudaStream_t s) {
+    cudaError_t e = cudaSuccess;
+    if (n <= 8) return n > 0 ? write_n<8>(dst, values, (int)n, s) : e;
+    for (int64_t i = 0; i < n && !e; i += 1024) e = write_n<1024>(dst + i, values + i, (int)std::min<int64_t>(1024, n - i), s);
+    return e;
 }
 
 cudaError_t launch_unpack(const MemberDev* members, const StencilTile* tiles, int ntiles, int large,

@@ -107,7 +107,7 @@ class QGParams:
         if any(isinstance(v, torch.Tensor) and v.requires_grad for v in vals):
             # keep the autograd connection to the parameters
             return torch.stack([torch.as_tensor(v, dtype=torch.float32, device=device).reshape(()) for v in vals])
-        return torch.tensor([float(v) for v in vals], dtype=torch.float32).to(device)  # one copy
+        return _device_vector([float(v) for v in vals], device)
 
 
 BaroclinicQGParams = QGParams
@@ -179,6 +179,18 @@ class Grid:
 # ---------------------------------------------------------------------------------------
 def _stream_handle(device) -> C.c_void_p:
     return C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+
+
+def _device_vector(vals, device) -> torch.Tensor:
+    """Host numbers as a float32 tensor on ``device``; on the current GPU in stream order, without
+    the wait of a copy from pageable memory (``qg_write``)."""
+    device = torch.device("cpu" if device is None else device)
+    if device.type != "cuda" or device.index not in (None, torch.cuda.current_device()):
+        return torch.tensor(vals, dtype=torch.float32).to(device)
+    out = torch.empty(len(vals), dtype=torch.float32, device=device)
+    check(_lib.lib().qg_write(C.c_void_p(out.data_ptr()), (C.c_float * len(vals))(*vals), len(vals),
+                              _stream_handle(out.device)), "qg_write")
+    return out
 
 
 def lsweep_classes(spec, rows: int) -> set:
@@ -914,8 +926,8 @@ class QGEnsemble:
         ts = [t for m in self.models for t in m._param_tensors()]
         if any(isinstance(t, torch.Tensor) and t.requires_grad for t in ts):
             return torch.cat([m._param_vector(device) for m in self.models])
-        # every member's parameters in one host-to-device copy
-        return torch.tensor([float(t) for t in ts], dtype=torch.float32).to(device)
+        # every member's parameters at once
+        return _device_vector([float(t) for t in ts], device)
 
     def pack(self, qs: Sequence[torch.Tensor]) -> torch.Tensor:
         if len(qs) != len(self.models):

@@ -24,7 +24,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .qg import SaveAt, Solution, SomaxModel, _solver_name, _stream_handle, check
+from .qg import SaveAt, Solution, SomaxModel, _device_vector, _solver_name, _stream_handle, check
 from .reparameterized import MultilayerSW2DState
 from .transforms import ModalTransform, StratificationProfile
 
@@ -350,8 +350,7 @@ class MultilayerShallowWater2D(SomaxModel):
 
     def _param_vector(self, device) -> torch.Tensor:
         p = self.params
-        return torch.tensor([float(p.lateral_viscosity), float(p.bottom_drag), float(p.wind_amplitude)],
-                            dtype=torch.float32, device=device)
+        return _device_vector([float(p.lateral_viscosity), float(p.bottom_drag), float(p.wind_amplitude)], device)
 
     def _param_tensor(self, device) -> torch.Tensor:
         """(nu, kappa, tau0) as a float32 device tensor that keeps the parameters' autograd graph."""
