@@ -421,14 +421,14 @@ cudaError_t launch_cols(const ColsArgs& a, int n_members, cudaStream_t s, bool p
 struct CapItem {
     int member, mode, r0;  // rows r0 .. r0 + kCapRows - 1 of C^-1 of one mode
 };
-constexpr int kCapRows = 32;
+constexpr int kCapRows = 8;
 std::vector<int> land_boundary(const qg_member_desc& d);
 bool capacitance_inverse(const qg_member_desc& d, const double* lam, int nl, const std::vector<int>& B,
                          std::vector<double>& cinv);
 // sigma = -C^-1 psi_hat[B] per (member, mode), written at B into the operand (and its FP32
 // copy) for the second solve
 cudaError_t launch_capacitance(const MemberDev* members, const CapItem* items, int n_items, const float* psi_hat,
-                               void* xa, int xa_fmt, float* xq, int64_t xplane, size_t smem, cudaStream_t s);
+                               void* xa, int xa_fmt, float* xq, int64_t xplane, size_t smem, cudaStream_t s, bool pdl);
 cudaError_t capacitance_init(size_t max_smem);
 constexpr int kMaxBoundary = 28000;  // boundary points per member (FP64 gather in shared memory)
 

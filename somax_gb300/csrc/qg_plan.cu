@@ -520,7 +520,7 @@ cudaError_t run_inversion(qg_plan* p, cudaStream_t s) {
     for (int c = 0; c < 1 + p->opts.refine_sweeps && !e; ++c) {
         e = timed(p, QG_K_OTHER, s, [&] {
             return launch_capacitance(p->md, p->cap_items, p->n_cap, p->XC, p->XA, p->op_fmt, p->XQ, p->xplane,
-                                      p->cap_smem, s);
+                                      p->cap_smem, s, use_pdl(p));
         });
         // a refinement sweep leaves its residual in the operand: rebuild it from the FP32
         // right-hand side (which holds the sources on B)
