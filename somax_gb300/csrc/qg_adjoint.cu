@@ -30,6 +30,7 @@
 #include <algorithm>
 
 #include "qg_internal.cuh"
+#include "qg_stencil_tile.cuh"
 
 namespace qg {
 
@@ -213,65 +214,74 @@ __global__ void __launch_bounds__(NT) k_vjp_tau(const MemberDev* __restrict__ me
 // Right-hand side of the adjoint solve in the GEMM operand format (plus its FP32 copy for the
 // refinement residual).  From the FP32 modal plane `rhs` when `psi_bar` is null, else
 // Cm2l^T Z psi_bar of a caller-packed layer cotangent (the VJP of the inversion).
-__global__ void __launch_bounds__(NT) k_vjp_operand(const MemberDev* __restrict__ members,
-                                                    const StencilTile* __restrict__ tiles, int TXr, int TYr,
-                                                    const float* __restrict__ rhs,
-                                                    const float* __restrict__ psi_bar, void* xa, int xa_fmt,
-                                                    float* xq, int64_t xplane) {
-    const StencilTile t = tiles[blockIdx.x];
-    const MemberDev& M = members[t.member];
-    const int nl = M.nl;
-    for (int c = threadIdx.x; c < TXr * TYr; c += NT) {
-        const int j = t.ty * TYr + c / TXr, i = t.tx * TXr + c % TXr;
-        if (j >= M.Ny || i >= M.Nx) continue;
-        float pb[kMaxLayers];
-        if (psi_bar) {
-            const bool zero = (!M.barotropic && on_ring(j, i, M.Ny, M.Nx)) || is_land(M.mask, M.Ny, M.Nx, j, i);
-            for (int l = 0; l < nl; ++l) pb[l] = zero ? 0.f : psi_bar[cidx(M, l, j, i)];
-        }
-        for (int m = 0; m < nl; ++m) {
-            const int64_t o = xidx(M, m, j, i);
-            float v = 0.f;
-            if (psi_bar) {
-                for (int l = 0; l < nl; ++l) v = fmaf(M.Cm2l[l * kMaxLayers + m], pb[l], v);
-            } else {
-                v = rhs[o];
-            }
-            if (xa_fmt == FMT_F32) {
-                static_cast<float*>(xa)[o] = v;
-            } else {
-                __nv_bfloat16* p = static_cast<__nv_bfloat16*>(xa);
-                const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-                p[o] = hi;
-                p[xplane + o] = __float2bfloat16_rn(v - __bfloat162float(hi));
-            }
-            if (xq) xq[o] = v;
-        }
-    }
+__global__ void __launch_bounds__(NT) k_vjp_operand(const MemberDev* members, const StencilTile* tiles, int TX, int TY,
+                                                    int parts, const float* rhs, const float* psi_bar, void* xa,
+                                                    int xa_fmt, float* xq, int64_t xplane) {
+    __shared__ MemberDev M;
+    const StencilTile t = tiles[blockIdx.x / (unsigned)parts];
+    st::load_member(&M, members + t.member);
+    __syncthreads();
+    pdl_wait();
+    pdl_launch_dependents();
+    st::with_layers(M.nl, [&](auto n) {
+        constexpr int NL = decltype(n)::value;
+        st::walk_cells<NL, NL <= 4 ? 4 : 2>(
+            M, t, TX, TY, parts,
+            [&](int j, int i, float(&x)[NL]) {
+#pragma unroll
+                for (int l = 0; l < NL; ++l) x[l] = psi_bar ? psi_bar[cidx(M, l, j, i)] : rhs[xidx(M, l, j, i)];
+            },
+            [&](int j, int i, float(&x)[NL]) {
+                const bool zero = (!M.barotropic && on_ring(j, i, M.Ny, M.Nx)) || is_land(M.mask, M.Ny, M.Nx, j, i);
+#pragma unroll
+                for (int m = 0; m < NL; ++m) {
+                    const int64_t o = xidx(M, m, j, i);
+                    float v = 0.f;
+                    if (!psi_bar)
+                        v = x[m];
+                    else if (!zero)
+#pragma unroll
+                        for (int l = 0; l < NL; ++l) v = fmaf(M.Cm2l[l * kMaxLayers + m], x[l], v);
+                    st::store_plane(xa, xa_fmt, xplane, o, v);
+                    if (xq) xq[o] = v;
+                }
+            });
+    });
 }
 
 // q_bar = B (direct + Cl2m^T x_bar) in caller packing, x_bar the adjoint solve's output.
-__global__ void __launch_bounds__(NT) k_vjp_finish(const MemberDev* __restrict__ members,
-                                                   const StencilTile* __restrict__ tiles, int TXr, int TYr,
-                                                   const float* __restrict__ direct,
-                                                   const float* __restrict__ xbar, int apply_bc,
-                                                   float* __restrict__ qbar) {
-    const StencilTile t = tiles[blockIdx.x];
-    const MemberDev& M = members[t.member];
-    const int nl = M.nl;
-    for (int c = threadIdx.x; c < TXr * TYr; c += NT) {
-        const int j = t.ty * TYr + c / TXr, i = t.tx * TXr + c % TXr;
-        if (j >= M.Ny || i >= M.Nx) continue;
-        // q of the ring (under the BC) and of land cells is not read by the forward
-        const bool zero = (apply_bc && on_ring(j, i, M.Ny, M.Nx)) || is_land(M.mask, M.Ny, M.Nx, j, i);
-        float xb[kMaxLayers];
-        for (int m = 0; m < nl; ++m) xb[m] = xbar[xidx(M, m, j, i)];
-        for (int l = 0; l < nl; ++l) {
-            float v = direct ? direct[xidx(M, l, j, i)] : 0.f;
-            for (int m = 0; m < nl; ++m) v = fmaf(M.Cl2m[m * kMaxLayers + l], xb[m], v);
-            qbar[cidx(M, l, j, i)] = zero ? 0.f : v;
-        }
-    }
+__global__ void __launch_bounds__(NT) k_vjp_finish(const MemberDev* members, const StencilTile* tiles, int TX, int TY,
+                                                   int parts, const float* direct, const float* xbar, int apply_bc,
+                                                   float* qbar) {
+    __shared__ MemberDev M;
+    const StencilTile t = tiles[blockIdx.x / (unsigned)parts];
+    st::load_member(&M, members + t.member);
+    __syncthreads();
+    pdl_wait();
+    pdl_launch_dependents();
+    st::with_layers(M.nl, [&](auto n) {
+        constexpr int NL = decltype(n)::value;
+        st::walk_cells<2 * NL, NL <= 2 ? 4 : 2>(
+            M, t, TX, TY, parts,
+            [&](int j, int i, float(&x)[2 * NL]) {
+#pragma unroll
+                for (int l = 0; l < NL; ++l) {
+                    x[l] = xbar[xidx(M, l, j, i)];
+                    x[NL + l] = direct ? direct[xidx(M, l, j, i)] : 0.f;
+                }
+            },
+            [&](int j, int i, float(&x)[2 * NL]) {
+                // q of the ring (under the BC) and of land cells is not read by the forward
+                const bool zero = (apply_bc && on_ring(j, i, M.Ny, M.Nx)) || is_land(M.mask, M.Ny, M.Nx, j, i);
+#pragma unroll
+                for (int l = 0; l < NL; ++l) {
+                    float v = x[NL + l];
+#pragma unroll
+                    for (int m = 0; m < NL; ++m) v = fmaf(M.Cl2m[m * kMaxLayers + l], x[m], v);
+                    qbar[cidx(M, l, j, i)] = zero ? 0.f : v;
+                }
+            });
+    });
 }
 
 __global__ void k_vjp_params(const double* __restrict__ pacc, int n, float* __restrict__ pbar) {
@@ -291,14 +301,15 @@ cudaError_t launch_vjp_stencil(const VjpArgs& v, cudaStream_t s) {
 }
 
 cudaError_t launch_vjp_operand(const VjpArgs& v, const float* psi_bar, cudaStream_t s) {
-    k_vjp_operand<<<v.ntiles, NT, 0, s>>>(v.members, v.tiles, v.tile_x, v.tile_y, v.rhs, psi_bar, v.xa, v.xa_fmt,
-                                          v.xq, v.xplane);
-    return cudaGetLastError();
+    const int parts = cell_parts(v.tile_x, v.ntiles);
+    return launch_k(k_vjp_operand, v.ntiles * parts, NT, 0, s, v.pdl, v.members, v.tiles, v.tile_x, v.tile_y, parts, v.rhs,
+                    psi_bar, v.xa, v.xa_fmt, v.xq, v.xplane);
 }
 
 cudaError_t launch_vjp_finish(const VjpArgs& v, const float* xbar, float* qbar, float* pbar, cudaStream_t s) {
-    k_vjp_finish<<<v.ntiles, NT, 0, s>>>(v.members, v.tiles, v.tile_x, v.tile_y, v.direct, xbar, v.apply_bc, qbar);
-    cudaError_t e = cudaGetLastError();
+    const int parts = cell_parts(v.tile_x, v.ntiles);
+    cudaError_t e = launch_k(k_vjp_finish, v.ntiles * parts, NT, 0, s, v.pdl, v.members, v.tiles, v.tile_x, v.tile_y,
+                             parts, v.direct, xbar, v.apply_bc, qbar);
     if (!e && pbar) {
         const int n = v.n_members * QG_NPARAMS;
         k_vjp_params<<<(n + 127) / 128, 128, 0, s>>>(v.pacc, n, pbar);

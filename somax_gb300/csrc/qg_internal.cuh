@@ -275,6 +275,7 @@ struct VjpArgs {
     int xa_fmt;
     float* xq;            // its FP32 copy for the refinement residual (may be null)
     int64_t xplane;
+    bool pdl;             // programmatic dependent launch
 };
 cudaError_t launch_vjp_stencil(const VjpArgs& v, cudaStream_t s);
 cudaError_t launch_vjp_operand(const VjpArgs& v, const float* psi_bar, cudaStream_t s);
@@ -499,5 +500,8 @@ int round_up(int v, int m);
 
 // stencil tile shapes (cells): small grids use 32 x 8, large ones 64 x 16
 constexpr int kTileSX = 32, kTileSY = 8, kTileLX = 64, kTileLY = 16;
+// CTAs per tile of the kernels that walk cells without a halo: the four passes of a large tile go to
+// four CTAs until a plan's tiles give every SM eight of them.
+constexpr int cell_parts(int tile_x, int ntiles) { return tile_x == kTileLX && ntiles < 8 * 152 ? 4 : 1; }
 
 }  // namespace qg

@@ -507,6 +507,7 @@ VjpArgs vjp_args(qg_plan* p) {
     v.xa_fmt = p->op_fmt;
     v.xq = p->XQ;
     v.xplane = p->xplane;
+    v.pdl = use_pdl(p);
     return v;
 }
 

@@ -22,51 +22,65 @@ using namespace st;
 // Pack: copy q (caller packing) into an internal plane (optionally zeroing its ring) and
 // write the layer->mode operand Cl2m q (BC applied when bc_operand) for the DST GEMMs.
 // ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(NTHREADS) k_prep(PrepArgs a) {
+__global__ void __launch_bounds__(NTHREADS) k_prep(PrepArgs a, int parts) {
     __shared__ MemberDev M;
-    const StencilTile t = a.tiles[blockIdx.x];
-    const int TX = a.tile_x, TY = a.tile_y;
+    const StencilTile t = a.tiles[blockIdx.x / (unsigned)parts];
     load_member(&M, a.members + t.member);
     __syncthreads();
     pdl_wait();
     pdl_launch_dependents();
-    const int nl = M.nl;
-    for (int c = threadIdx.x; c < TX * TY; c += blockDim.x) {
-        const int j = t.ty * TY + c / TX, i = t.tx * TX + c % TX;
-        if (j >= M.Ny || i >= M.Nx) continue;
-        const bool ring = on_ring(j, i, M.Ny, M.Nx);
-        const bool land = is_land(M, j, i);  // q reads as zero on land
-        float v[kMaxLayers];
-        for (int l = 0; l < nl; ++l) {
-            const float x = a.q[caller_idx(M, l, j, i)];
-            if (a.copy) a.copy[xrow_idx(M, l, j, i)] = (a.zero_ring_copy && (ring || land)) ? 0.f : x;
-            v[l] = ((a.bc_operand && ring) || land) ? 0.f : x;
-        }
-        if (!a.xa) continue;
-        for (int m = 0; m < nl; ++m) {
-            float s = 0.f;
-            for (int l = 0; l < nl; ++l) s = fmaf(M.Cl2m[m * kMaxLayers + l], v[l], s);
-            store_plane(a.xa, a.xa_fmt, a.xplane, xrow_idx(M, m, j, i), s);
-            if (a.xq) a.xq[xrow_idx(M, m, j, i)] = s;
-        }
-    }
+    with_layers(M.nl, [&](auto n) {
+        constexpr int NL = decltype(n)::value;
+        walk_cells<NL, NL <= 4 ? 4 : 2>(
+            M, t, a.tile_x, a.tile_y, parts,
+            [&](int j, int i, float(&x)[NL]) {
+#pragma unroll
+                for (int l = 0; l < NL; ++l) x[l] = a.q[caller_idx(M, l, j, i)];
+            },
+            [&](int j, int i, float(&x)[NL]) {
+                const bool ring = on_ring(j, i, M.Ny, M.Nx);
+                const bool land = is_land(M, j, i);  // q reads as zero on land
+#pragma unroll
+                for (int l = 0; l < NL; ++l) {
+                    if (a.copy) a.copy[xrow_idx(M, l, j, i)] = (a.zero_ring_copy && (ring || land)) ? 0.f : x[l];
+                    x[l] = ((a.bc_operand && ring) || land) ? 0.f : x[l];
+                }
+                if (!a.xa) return;
+#pragma unroll
+                for (int m = 0; m < NL; ++m) {
+                    float s = 0.f;
+#pragma unroll
+                    for (int l = 0; l < NL; ++l) s = fmaf(M.Cl2m[m * kMaxLayers + l], x[l], s);
+                    store_plane(a.xa, a.xa_fmt, a.xplane, xrow_idx(M, m, j, i), s);
+                    if (a.xq) a.xq[xrow_idx(M, m, j, i)] = s;
+                }
+            });
+    });
 }
 
 // Unpack: internal plane -> caller packing (every cell, ring included).
 __global__ void __launch_bounds__(NTHREADS) k_unpack(const MemberDev* __restrict__ members,
-                                                     const StencilTile* __restrict__ tiles, int TX, int TY,
-                                                     const float* __restrict__ src, float* __restrict__ q) {
+                                                     const StencilTile* __restrict__ tiles, int TX, int TY, int parts,
+                                                     const float* src, float* q) {
     __shared__ MemberDev M;
-    const StencilTile t = tiles[blockIdx.x];
+    const StencilTile t = tiles[blockIdx.x / (unsigned)parts];
     load_member(&M, members + t.member);
     __syncthreads();
     pdl_wait();
     pdl_launch_dependents();
-    for (int c = threadIdx.x; c < TX * TY; c += blockDim.x) {
-        const int j = t.ty * TY + c / TX, i = t.tx * TX + c % TX;
-        if (j >= M.Ny || i >= M.Nx) continue;
-        for (int l = 0; l < M.nl; ++l) q[caller_idx(M, l, j, i)] = src[xrow_idx(M, l, j, i)];
-    }
+    with_layers(M.nl, [&](auto n) {
+        constexpr int NL = decltype(n)::value;
+        walk_cells<NL, NL <= 4 ? 4 : 2>(
+            M, t, TX, TY, parts,
+            [&](int j, int i, float(&x)[NL]) {
+#pragma unroll
+                for (int l = 0; l < NL; ++l) x[l] = src[xrow_idx(M, l, j, i)];
+            },
+            [&](int j, int i, float(&x)[NL]) {
+#pragma unroll
+                for (int l = 0; l < NL; ++l) q[caller_idx(M, l, j, i)] = x[l];
+            });
+    });
 }
 
 // ---------------------------------------------------------------------------------------
@@ -76,36 +90,49 @@ __global__ void __launch_bounds__(NTHREADS) k_unpack(const MemberDev* __restrict
 // solve.  The ring is combined like every other cell; stage inputs are read with the BC, and
 // the final combination's ring is y0 + dt * wind as in the fused Shu-Osher stencil.
 // ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(NTHREADS) k_rk_combine(RkCombineArgs a) {
+__global__ void __launch_bounds__(NTHREADS) k_rk_combine(RkCombineArgs a, int parts) {
     __shared__ MemberDev M;
-    const StencilTile t = a.tiles[blockIdx.x];
+    const StencilTile t = a.tiles[blockIdx.x / (unsigned)parts];
     load_member(&M, a.members + t.member);
     __syncthreads();
     pdl_wait();
     pdl_launch_dependents();
-    const int nl = M.nl, TX = a.tile_x, TY = a.tile_y;
-    for (int c = threadIdx.x; c < TX * TY; c += blockDim.x) {
-        const int j = t.ty * TY + c / TX, i = t.tx * TX + c % TX;
-        if (j >= M.Ny || i >= M.Nx) continue;
-        const bool zero = on_ring(j, i, M.Ny, M.Nx) || is_land(M, j, i);
-        float v[kMaxLayers];
-        for (int l = 0; l < nl; ++l) {
-            const int64_t ci = caller_idx(M, l, j, i);
-            float acc = 0.f;
-            for (int s = 0; s < a.n_k; ++s)
-                if (a.coef[s] != 0.f) acc = fmaf(a.coef[s], a.k[(int64_t)s * a.kplane + ci], acc);
-            const int64_t xi = xrow_idx(M, l, j, i);
-            v[l] = a.y0[xi] + a.dt * acc;
-            a.out[xi] = v[l];
-        }
-        for (int m = 0; m < nl; ++m) {
-            float sum = 0.f;
-            if (!zero)
-                for (int l = 0; l < nl; ++l) sum = fmaf(M.Cl2m[m * kMaxLayers + l], v[l], sum);
-            store_plane(a.xa, a.xa_fmt, a.xplane, xrow_idx(M, m, j, i), sum);
-            if (a.xq) a.xq[xrow_idx(M, m, j, i)] = sum;
-        }
-    }
+    with_layers(M.nl, [&](auto n) {
+        constexpr int NL = decltype(n)::value;
+        walk_cells<NL, NL <= 2 ? 4 : NL <= 4 ? 2 : 1>(
+            M, t, a.tile_x, a.tile_y, parts,
+            [&](int j, int i, float(&v)[NL]) {
+                const int64_t ci = caller_idx(M, 0, j, i), cl = (int64_t)M.Ny * M.Nx;
+                float acc[NL];
+#pragma unroll
+                for (int l = 0; l < NL; ++l) {
+                    acc[l] = 0.f;
+                    v[l] = a.y0[xrow_idx(M, l, j, i)];
+                }
+#pragma unroll
+                for (int s = 0; s < kMaxButcher; ++s)
+                    if (s < a.n_k && a.coef[s] != 0.f)
+#pragma unroll
+                        for (int l = 0; l < NL; ++l)
+                            acc[l] = fmaf(a.coef[s], a.k[(int64_t)s * a.kplane + ci + l * cl], acc[l]);
+#pragma unroll
+                for (int l = 0; l < NL; ++l) v[l] += a.dt * acc[l];
+            },
+            [&](int j, int i, float(&v)[NL]) {
+                const bool zero = on_ring(j, i, M.Ny, M.Nx) || is_land(M, j, i);
+#pragma unroll
+                for (int l = 0; l < NL; ++l) a.out[xrow_idx(M, l, j, i)] = v[l];
+#pragma unroll
+                for (int m = 0; m < NL; ++m) {
+                    float sum = 0.f;
+                    if (!zero)
+#pragma unroll
+                        for (int l = 0; l < NL; ++l) sum = fmaf(M.Cl2m[m * kMaxLayers + l], v[l], sum);
+                    store_plane(a.xa, a.xa_fmt, a.xplane, xrow_idx(M, m, j, i), sum);
+                    if (a.xq) a.xq[xrow_idx(M, m, j, i)] = sum;
+                }
+            });
+    });
 }
 
 // ---------------------------------------------------------------------------------------
@@ -113,27 +140,32 @@ __global__ void __launch_bounds__(NTHREADS) k_rk_combine(RkCombineArgs a) {
 // ---------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(NTHREADS) k_mode_to_layer(const MemberDev* __restrict__ members,
                                                             const StencilTile* __restrict__ tiles, int TX, int TY,
-                                                            const float* __restrict__ psi_hat,
-                                                            float* __restrict__ psi) {
+                                                            int parts, const float* psi_hat, float* psi) {
     __shared__ MemberDev M;
-    const StencilTile t = tiles[blockIdx.x];
+    const StencilTile t = tiles[blockIdx.x / (unsigned)parts];
     load_member(&M, members + t.member);
     __syncthreads();
     pdl_wait();
     pdl_launch_dependents();
-    const int nl = M.nl;
-    for (int c = threadIdx.x; c < TX * TY; c += blockDim.x) {
-        const int j = t.ty * TY + c / TX, i = t.tx * TX + c % TX;
-        if (j >= M.Ny || i >= M.Nx) continue;
-        const bool zero = (!M.barotropic && on_ring(j, i, M.Ny, M.Nx)) || is_land(M, j, i);
-        float ph[kMaxLayers];
-        for (int m = 0; m < nl; ++m) ph[m] = psi_hat[xrow_idx(M, m, j, i)];
-        for (int l = 0; l < nl; ++l) {
-            float p = 0.f;
-            for (int m = 0; m < nl; ++m) p = fmaf(M.Cm2l[l * kMaxLayers + m], ph[m], p);
-            psi[caller_idx(M, l, j, i)] = zero ? 0.f : p;
-        }
-    }
+    with_layers(M.nl, [&](auto n) {
+        constexpr int NL = decltype(n)::value;
+        walk_cells<NL, NL <= 4 ? 4 : 2>(
+            M, t, TX, TY, parts,
+            [&](int j, int i, float(&x)[NL]) {
+#pragma unroll
+                for (int m = 0; m < NL; ++m) x[m] = psi_hat[xrow_idx(M, m, j, i)];
+            },
+            [&](int j, int i, float(&x)[NL]) {
+                const bool zero = (!M.barotropic && on_ring(j, i, M.Ny, M.Nx)) || is_land(M, j, i);
+#pragma unroll
+                for (int l = 0; l < NL; ++l) {
+                    float p = 0.f;
+#pragma unroll
+                    for (int m = 0; m < NL; ++m) p = fmaf(M.Cm2l[l * kMaxLayers + m], x[m], p);
+                    psi[caller_idx(M, l, j, i)] = zero ? 0.f : p;
+                }
+            });
+    });
 }
 
 // ---------------------------------------------------------------------------------------
@@ -284,31 +316,34 @@ __global__ void __launch_bounds__(NTHREADS) k_project_q_vjp(const MemberDev* __r
 // operator the DST-I solve inverts).  qm is the FP32 modal right-hand side.
 // ---------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(NTHREADS) k_residual(const MemberDev* __restrict__ members,
-                                                       const StencilTile* __restrict__ tiles, int TX, int TY,
-                                                       const float* __restrict__ qm,
-                                                       const float* __restrict__ psi_hat,
-                                                       void* out, int out_fmt, int64_t xplane) {
+                                                       const StencilTile* __restrict__ tiles, int TX, int TY, int parts,
+                                                       const float* qm, const float* psi_hat, void* out, int out_fmt,
+                                                       int64_t xplane) {
     __shared__ MemberDev M;
-    const StencilTile t = tiles[blockIdx.x];
+    const StencilTile t = tiles[blockIdx.x / (unsigned)parts];
     load_member(&M, members + t.member);
     __syncthreads();
     pdl_wait();
     pdl_launch_dependents();
-    const int nl = M.nl, Ny = M.Ny, Nx = M.Nx;
-    for (int c = threadIdx.x; c < TX * TY; c += blockDim.x) {
-        const int j = t.ty * TY + c / TX, i = t.tx * TX + c % TX;
-        if (j >= Ny || i >= Nx) continue;
-        for (int m = 0; m < nl; ++m) {
-            auto P = [&](int jj, int ii) {
-                return (jj < 0 || jj >= Ny || ii < 0 || ii >= Nx) ? 0.f : psi_hat[xrow_idx(M, m, jj, ii)];
-            };
-            const float c0 = P(j, i);
-            const float lap = (P(j, i + 1) - 2.f * c0 + P(j, i - 1)) * M.inv_dx2 +
-                              (P(j + 1, i) - 2.f * c0 + P(j - 1, i)) * M.inv_dy2;
-            const float r = qm[xrow_idx(M, m, j, i)] - (lap - M.lam[m] * c0);
-            store_plane(out, out_fmt, xplane, xrow_idx(M, m, j, i), r);
-        }
-    }
+    with_layers(M.nl, [&](auto n) {
+        constexpr int NL = decltype(n)::value;
+        walk_cells<NL, NL <= 2 ? 2 : 1>(
+            M, t, TX, TY, parts,
+            [&](int j, int i, float(&r)[NL]) {
+#pragma unroll
+                for (int m = 0; m < NL; ++m) {
+                    const float* p = psi_hat + xrow_idx(M, m, j, i);
+                    const float c0 = p[0], e = i + 1 < M.Nx ? p[1] : 0.f, w = i > 0 ? p[-1] : 0.f;
+                    const float no = j + 1 < M.Ny ? p[M.Px] : 0.f, so = j > 0 ? p[-M.Px] : 0.f;
+                    const float lap = (e - 2.f * c0 + w) * M.inv_dx2 + (no - 2.f * c0 + so) * M.inv_dy2;
+                    r[m] = qm[xrow_idx(M, m, j, i)] - (lap - M.lam[m] * c0);
+                }
+            },
+            [&](int j, int i, float(&r)[NL]) {
+#pragma unroll
+                for (int m = 0; m < NL; ++m) store_plane(out, out_fmt, xplane, xrow_idx(M, m, j, i), r[m]);
+            });
+    });
 }
 
 // ---------------------------------------------------------------------------------------
@@ -548,11 +583,13 @@ cudaError_t stencil_encode_maps(const MemberDev& M, const float* const planes[4]
 }
 
 cudaError_t launch_prep(const PrepArgs& a, int ntiles, cudaStream_t s, bool pdl) {
-    return launch_k(k_prep, ntiles, NTHREADS, 0, s, pdl, a);
+    const int parts = cell_parts(a.tile_x, ntiles);
+    return launch_k(k_prep, ntiles * parts, NTHREADS, 0, s, pdl, a, parts);
 }
 
 cudaError_t launch_rk_combine(const RkCombineArgs& a, int ntiles, cudaStream_t s, bool pdl) {
-    return launch_k(k_rk_combine, ntiles, NTHREADS, 0, s, pdl, a);
+    const int parts = cell_parts(a.tile_x, ntiles);
+    return launch_k(k_rk_combine, ntiles * parts, NTHREADS, 0, s, pdl, a, parts);
 }
 
 namespace {
@@ -585,14 +622,14 @@ cudaError_t launch_write(float* dst, const float* values, int64_t n, cudaStream_
 
 cudaError_t launch_unpack(const MemberDev* members, const StencilTile* tiles, int ntiles, int large,
                           const float* src, float* q, cudaStream_t s, bool pdl) {
-    return launch_k(k_unpack, ntiles, NTHREADS, 0, s, pdl, members, tiles, large ? TileL::TX : TileS::TX,
-                    large ? TileL::TY : TileS::TY, src, q);
+    const int tx = large ? TileL::TX : TileS::TX, ty = large ? TileL::TY : TileS::TY, parts = cell_parts(tx, ntiles);
+    return launch_k(k_unpack, ntiles * parts, NTHREADS, 0, s, pdl, members, tiles, tx, ty, parts, src, q);
 }
 
 cudaError_t launch_mode_to_layer(const MemberDev* members, const StencilTile* tiles, int ntiles, int large,
                                  const float* psi_hat, float* psi, cudaStream_t s, bool pdl) {
-    return launch_k(k_mode_to_layer, ntiles, NTHREADS, 0, s, pdl, members, tiles, large ? TileL::TX : TileS::TX,
-                    large ? TileL::TY : TileS::TY, psi_hat, psi);
+    const int tx = large ? TileL::TX : TileS::TX, ty = large ? TileL::TY : TileS::TY, parts = cell_parts(tx, ntiles);
+    return launch_k(k_mode_to_layer, ntiles * parts, NTHREADS, 0, s, pdl, members, tiles, tx, ty, parts, psi_hat, psi);
 }
 
 cudaError_t launch_project_q(const MemberDev* members, const StencilTile* tiles, int ntiles, int large,
@@ -622,8 +659,9 @@ cudaError_t launch_project_q_vjp(const MemberDev* members, const StencilTile* ti
 cudaError_t launch_residual(const MemberDev* members, const StencilTile* tiles, int ntiles, int large,
                             const float* qm, const float* psi_hat, void* out, int out_fmt,
                             int64_t xplane, cudaStream_t s, bool pdl) {
-    return launch_k(k_residual, ntiles, NTHREADS, 0, s, pdl, members, tiles, large ? TileL::TX : TileS::TX,
-                    large ? TileL::TY : TileS::TY, qm, psi_hat, out, out_fmt, xplane);
+    const int tx = large ? TileL::TX : TileS::TX, ty = large ? TileL::TY : TileS::TY, parts = cell_parts(tx, ntiles);
+    return launch_k(k_residual, ntiles * parts, NTHREADS, 0, s, pdl, members, tiles, tx, ty, parts, qm, psi_hat, out,
+                    out_fmt, xplane);
 }
 
 cudaError_t launch_diag_acc(const MemberDev* members, const StencilTile* tiles, int ntiles, int large,

@@ -9,6 +9,8 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include <type_traits>
+
 #include "qg_device.cuh"
 #include "qg_internal.cuh"
 
@@ -76,6 +78,52 @@ __device__ __forceinline__ void store_plane(void* base, int fmt, int64_t plane_e
         __nv_bfloat16* p = static_cast<__nv_bfloat16*>(base);
         p[idx] = hi;
         p[plane_elems + idx] = lo;
+    }
+}
+
+// f(integral constant NL) for a member of nl layers: loops over layers with compile-time bounds.
+template <class F>
+__device__ __forceinline__ void with_layers(int nl, F&& f) {
+    static_assert(kMaxLayers == 8, "a case per layer count");
+    switch (nl) {
+        case 1: f(std::integral_constant<int, 1>{}); break;
+        case 2: f(std::integral_constant<int, 2>{}); break;
+        case 3: f(std::integral_constant<int, 3>{}); break;
+        case 4: f(std::integral_constant<int, 4>{}); break;
+        case 5: f(std::integral_constant<int, 5>{}); break;
+        case 6: f(std::integral_constant<int, 6>{}); break;
+        case 7: f(std::integral_constant<int, 7>{}); break;
+        default: f(std::integral_constant<int, 8>{}); break;
+    }
+}
+
+// The cells of a tile for a kernel without a halo: NL values x of a cell from load(j, i, x), then
+// use(j, i, x).  Bound: HBM on large plans, latency on small ones.  Loops over a layer count known
+// at run time kept one or two loads of a thread in flight; here every load of UNR cells, all layers,
+// is issued before the first store.  `parts` CTAs share a tile (cell_parts).
+template <int NL, int UNR, class Load, class Use>
+__device__ __forceinline__ void walk_cells(const MemberDev& M, const StencilTile& t, int TX, int TY, int parts,
+                                           Load&& load, Use&& use) {
+    const int sh = TX == kTileLX ? 6 : 5, step = NTHREADS * parts;
+    static_assert(kTileLX == 64 && kTileSX == 32, "tile columns by shift");
+    for (int c0 = threadIdx.x + (int)(blockIdx.x % (unsigned)parts) * NTHREADS; c0 < TX * TY; c0 += UNR * step) {
+        float x[UNR][NL];
+        auto at = [&](int u, int& j, int& i) {
+            const int c = c0 + u * step;
+            j = t.ty * TY + (c >> sh);
+            i = t.tx * TX + (c & (TX - 1));
+            return c < TX * TY && j < M.Ny && i < M.Nx;
+        };
+#pragma unroll
+        for (int u = 0; u < UNR; ++u) {
+            int j, i;
+            if (at(u, j, i)) load(j, i, x[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < UNR; ++u) {
+            int j, i;
+            if (at(u, j, i)) use(j, i, x[u]);
+        }
     }
 }
 
