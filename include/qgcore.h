@@ -273,9 +273,9 @@ int qg_kernel_stats(qg_plan* plan, int kclass, double* total_ms, int64_t* launch
 /* The plan's tuned choice: *variant = the stencil the multi-launch path runs; ms[k] (k < n)
    the autotuner's time of one stage with variant k in ms (-1 when not measured). */
 int qg_plan_tuning(const qg_plan* plan, int* variant, float* ms, int n);
-/* The tensor-core DST passes' output tile width the autotuner kept (144, 80, 48, 32 or 16
-   columns; 64 for the FP32 CUDA-core passes) and the time of the four passes it measured
-   with each width in ms (ms[0..4] in that order; -1 when not measured). */
+/* The tensor-core DST passes' output tile width the autotuner kept (144, 80, 48, 32, 16, 176,
+   208 or 256 columns; 64 for the FP32 CUDA-core passes) and the time of the four passes it
+   measured with each width in ms (ms[0..7] in that order; -1 when not measured). */
 int qg_plan_gemm_tuning(const qg_plan* plan, int* tile_n, float* ms, int n);
 /* The stepping engine qg_step uses for Heun / SSP-RK3: *cluster_ctas = the CTAs of one
    member's cluster when the cluster-resident engine runs (all members alike in layers and

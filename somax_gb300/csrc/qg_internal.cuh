@@ -291,7 +291,7 @@ const Tableau* swm_tableau(int scheme);
 
 // host: cuTensorMapEncodeTiled through the driver entry point (no libcuda link needed)
 cudaError_t tmap_encode(void* map, int bf16, int rank, const void* base, const uint64_t* dims,
-                        const uint64_t* strides_bytes, const uint32_t* box, int swizzle128);
+                        const uint64_t* strides_bytes, const uint32_t* box, int swizzle);  // bytes: 0, 64, 128
 
 struct GemmArgs {
     const MemberDev* members;
@@ -315,7 +315,7 @@ struct PersistArgs {
     const StencilTile* st;
     int n_gx, n_gy, n_st, max_nl;
     int tile_n;               // DST GEMM output tile width (<= TC_BN, a multiple of 16)
-    const void* tc_maps;
+    const void* tc_maps;      // for that width
     const void* st_maps;
     void *XA, *YA, *YB, *XB;  // operand-format planes
     float* XC;                // psi_hat
@@ -335,7 +335,7 @@ struct PersistArgs {
     unsigned* bar_gen;
     long long bar_wait;       // clock64 cycles a CTA waits at the grid barrier before giving up
 };
-size_t persistent_smem_bytes(int precision, int max_nl, int large, PersistArgs* a);
+size_t persistent_smem_bytes(int max_nl, int large, PersistArgs* a);
 cudaError_t persistent_init();
 cudaError_t launch_persistent(const PersistArgs& a, int grid, int precision, cudaStream_t s);
 // multi-tile stand-alone launches (the graph-captured multi-launch path)
@@ -343,7 +343,7 @@ cudaError_t launch_gemm_mt(const PersistArgs& a, int pass, int grid, int precisi
 cudaError_t launch_stencil_mt(const StencilArgs& sa, int n_st, int grid, int max_nl, int large, cudaStream_t s,
                               bool pdl);
 int stencil_mt_blocks_per_sm(int max_nl, int large);  // 4 CUtensorMap per (member, pass)
-cudaError_t gemm_tc_encode(const MemberDev& M, int pass, const void* a_plane, int64_t a_plane_elems, int prec,
+cudaError_t gemm_tc_encode(const MemberDev& M, int pass, const void* a_plane, int64_t a_plane_elems, int prec, int bn,
                            void* out);
 // FP32 CUDA-core passes (qg_gemm_simt.cu): tile shapes, from the largest to the smallest; a
 // pass over members with N columns has simt_row_tiles(shape, rows) x simt_col_tiles(shape, N)

@@ -81,22 +81,24 @@ __device__ bool grid_sync(unsigned* count, unsigned* gen, int* flags, volatile i
 struct Counters {
     uint32_t prod_kb = 0;   // k-blocks issued by the producer
     uint32_t mma_kb = 0;    // k-blocks consumed by the MMA thread
+    int slot = 0;           // ring slot and pass of the next k-block (producer, MMA thread)
+    uint32_t lap = 0;
     uint32_t mma_tiles = 0; // accumulators filled
     uint32_t epi_tiles = 0; // accumulators drained
     uint32_t st_use[2] = {0, 0};  // stencil box loads per buffer
 };
 
 struct Shared {
-    uint64_t full[4], empty[4], tfull[2], tempty[2], sbar[2];
+    uint64_t full[TC_MAX_STAGES], empty[TC_MAX_STAGES], tfull[2], tempty[2], sbar[2];
     uint32_t tmem_slot;
     int abort;
     int issued, consumed, committed;  // for draining after an abort
     MemberDev M;                      // constants of the current stencil tile
 };
 
-template <int PREC, int PASS, int EPI = 4>
+template <int PREC, int ROW, int PASS, int EPI = 4>
 __device__ void gemm_phase(const PersistArgs& a, uint8_t* smem, Shared& sh, uint32_t tmem, Counters& c) {
-    using C = TcCfg<PREC>;
+    using C = TcCfg<PREC, ROW>;
     constexpr bool xin = pass_xin(PASS);
     const GemmTile* tiles = xin ? a.gx : a.gy;
     const int n = xin ? a.n_gx : a.n_gy;
@@ -105,6 +107,15 @@ __device__ void gemm_phase(const PersistArgs& a, uint8_t* smem, Shared& sh, uint
     const TcMaps* maps = static_cast<const TcMaps*>(a.tc_maps);
     volatile int* abort = &sh.abort;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int stages = tc_stages<PREC, ROW>(a.tile_n), stage_bytes = tc_stage_bytes<PREC, ROW>(a.tile_n);
+    constexpr int a_bytes = TC_BM * ROW;
+    const int b_bytes = a.tile_n * ROW;
+    auto next_slot = [&] {
+        if (++c.slot == stages) {
+            c.slot = 0;
+            c.lap ^= 1;
+        }
+    };
 
     if (warp == 0 && lane == 0) {
         proxy_fence_shared();  // the stencil phase wrote this shared memory with generic stores
@@ -115,16 +126,17 @@ __device__ void gemm_phase(const PersistArgs& a, uint8_t* smem, Shared& sh, uint
             const TcGeom g = tc_geom<PASS>(a.members[tl.member], a.xplane, a.yplane);
             const int nkb = (g.K + C::BK - 1) / C::BK;
             for (int kb = 0; kb < nkb; ++kb) {
-                const int s = c.prod_kb % C::STAGES;
-                if (!mbar_wait(&sh.empty[s], ((c.prod_kb / C::STAGES) & 1) ^ 1, abort)) break;
-                uint8_t* stg = smem + s * tc_stage_bytes<PREC>();
-                mbar_expect_tx(&sh.full[s], tc_stage_bytes<PREC>());
+                const int s = c.slot;
+                if (!mbar_wait(&sh.empty[s], c.lap ^ 1, abort)) break;
+                uint8_t* stg = smem + s * stage_bytes;
+                mbar_expect_tx(&sh.full[s], stage_bytes);
                 for (int q = 0; q < C::NA; ++q)
-                    tma_load_2d(stg + q * tc_tile_a_bytes<PREC>(), &tm->a[q], &sh.full[s], kb * C::BK, tl.mt * TC_BM);
+                    tma_load_2d(stg + q * a_bytes, &tm->a[q], &sh.full[s], kb * C::BK, tl.mt * TC_BM);
                 for (int q = 0; q < C::NB; ++q)
-                    tma_load_2d(stg + C::NA * tc_tile_a_bytes<PREC>() + q * tc_tile_b_bytes<PREC>(), &tm->b[q],
-                                &sh.full[s], kb * C::BK, tl.nt * a.tile_n);
+                    tma_load_2d(stg + C::NA * a_bytes + q * b_bytes, &tm->b[q], &sh.full[s], kb * C::BK,
+                                tl.nt * a.tile_n);
                 sh.issued = (int)++c.prod_kb;
+                next_slot();
             }
         }
     } else if (warp == 1 && lane == 0) {
@@ -139,14 +151,15 @@ __device__ void gemm_phase(const PersistArgs& a, uint8_t* smem, Shared& sh, uint
             const uint32_t acc = tmem + buf * TC_TMEM_BUF;
             const int width = tc_tile_width(g.Nn, tl.nt, a.tile_n);
             for (int kb = 0; kb < nkb; ++kb) {
-                const int s = c.mma_kb % C::STAGES;
-                if (!mbar_wait(&sh.full[s], (c.mma_kb / C::STAGES) & 1, abort)) break;
+                const int s = c.slot;
+                if (!mbar_wait(&sh.full[s], c.lap, abort)) break;
                 tc_fence_after();
-                const uint32_t sa = su32(smem + s * tc_stage_bytes<PREC>());
+                const uint32_t sa = su32(smem + s * stage_bytes);
                 const int ksteps = (min(C::BK, g.K - kb * C::BK) + C::UMMA_K - 1) / C::UMMA_K;
-                tc_mma_kblock<PREC>(acc, sa, sa + C::NA * tc_tile_a_bytes<PREC>(), kb == 0, ksteps, width);
+                tc_mma_kblock<PREC, ROW>(acc, sa, sa + C::NA * a_bytes, b_bytes, kb == 0, ksteps, width);
                 tc_commit(&sh.empty[s]);
                 sh.consumed = (int)++c.mma_kb;
+                next_slot();
             }
             tc_commit(&sh.tfull[buf]);
             sh.committed = (int)++c.mma_tiles;
@@ -251,9 +264,9 @@ __device__ void stencil_phase(const PersistArgs& a, int k, uint8_t* smem, Shared
     stencil_tiles<T>(sa, a.n_st, smem, a.slot_bytes, a.lap_offset, a.st_nbuf, sh, c);
 }
 
-__device__ void init_shared(Shared& sh, int stages, int epi_warps = 4) {
+__device__ void init_shared(Shared& sh, int epi_warps = 4) {
     if (threadIdx.x == 0) {
-        for (int s = 0; s < stages; ++s) {
+        for (int s = 0; s < TC_MAX_STAGES; ++s) {
             mbar_init(&sh.full[s], 1);
             mbar_init(&sh.empty[s], 1);
         }
@@ -270,10 +283,9 @@ __device__ void init_shared(Shared& sh, int stages, int epi_warps = 4) {
 
 // After an abort: drain TMA copies issued but not consumed, then the MMAs of the last
 // committed accumulator, so that shared memory and TMEM are quiet before the CTA exits.
-template <int STAGES>
-__device__ void drain_after_abort(Shared& sh) {
+__device__ void drain_after_abort(Shared& sh, int stages) {
     if (sh.abort && threadIdx.x == 0) {
-        for (int kb = sh.consumed; kb < sh.issued; ++kb) mbar_drain(&sh.full[kb % STAGES], (kb / STAGES) & 1);
+        for (int kb = sh.consumed; kb < sh.issued; ++kb) mbar_drain(&sh.full[kb % stages], (kb / stages) & 1);
         if (sh.committed > 0) {
             const int t = sh.committed - 1;
             mbar_drain(&sh.tfull[t & 1], (t >> 1) & 1);
@@ -284,13 +296,12 @@ __device__ void drain_after_abort(Shared& sh) {
 // One DST-I GEMM pass as its own launch: output tiles of all members round-robin over
 // min(tiles, SMs) CTAs, two TMEM accumulators so a tile's epilogue overlaps the next
 // tile's MMAs.
-template <int PREC, int PASS>
+template <int PREC, int ROW, int PASS>
 __global__ void __launch_bounds__(PT_GEMM, 1) k_gemm_mt(PersistArgs a) {
-    using C = TcCfg<PREC>;
     extern __shared__ uint8_t smem_raw[];
     __shared__ Shared sh;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    init_shared(sh, C::STAGES, GEMM_EPI_WARPS);
+    init_shared(sh, GEMM_EPI_WARPS);
     if ((threadIdx.x >> 5) == 1) tc_alloc(&sh.tmem_slot, TC_TMEM_COLS);
     tc_fence_before();
     __syncthreads();
@@ -299,9 +310,9 @@ __global__ void __launch_bounds__(PT_GEMM, 1) k_gemm_mt(PersistArgs a) {
     pdl_wait();
     pdl_launch_dependents();
     Counters c;
-    gemm_phase<PREC, PASS, GEMM_EPI_WARPS>(a, smem, sh, tmem, c);
+    gemm_phase<PREC, ROW, PASS, GEMM_EPI_WARPS>(a, smem, sh, tmem, c);
     __syncthreads();
-    drain_after_abort<C::STAGES>(sh);
+    drain_after_abort(sh, tc_stages<PREC, ROW>(a.tile_n));
     tc_fence_before();
     __syncthreads();
     if ((threadIdx.x >> 5) == 1) {
@@ -318,7 +329,7 @@ __global__ void __launch_bounds__(PT, 3) k_stencil_mt(StencilArgs sa, int n_st, 
     extern __shared__ uint8_t smem_raw[];
     __shared__ Shared sh;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    init_shared(sh, 0);
+    init_shared(sh);
     __syncthreads();
     pdl_wait();
     pdl_launch_dependents();
@@ -328,12 +339,11 @@ __global__ void __launch_bounds__(PT, 3) k_stencil_mt(StencilArgs sa, int n_st, 
 
 template <int PREC, class T>
 __global__ void __launch_bounds__(PT, 1) k_persistent(PersistArgs a) {
-    using C = TcCfg<PREC>;
     extern __shared__ uint8_t smem_raw[];
     __shared__ Shared sh;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int warp = threadIdx.x >> 5;
-    init_shared(sh, C::STAGES);
+    init_shared(sh);
     if (warp == 1) tc_alloc(&sh.tmem_slot, TC_TMEM_COLS);
     tc_fence_before();
     __syncthreads();
@@ -344,13 +354,13 @@ __global__ void __launch_bounds__(PT, 1) k_persistent(PersistArgs a) {
 
     for (int step = 0; step < a.n_steps; ++step) {
         for (int k = 0; k < a.n_stages; ++k) {
-            gemm_phase<PREC, G1_FWD_X>(a, smem, sh, tmem, c);
+            gemm_phase<PREC, 128, G1_FWD_X>(a, smem, sh, tmem, c);
             if (!grid_sync(a.bar_count, a.bar_gen, a.flags, abort, a.bar_wait)) goto done;
-            gemm_phase<PREC, G2_FWD_Y>(a, smem, sh, tmem, c);
+            gemm_phase<PREC, 128, G2_FWD_Y>(a, smem, sh, tmem, c);
             if (!grid_sync(a.bar_count, a.bar_gen, a.flags, abort, a.bar_wait)) goto done;
-            gemm_phase<PREC, G3_INV_X>(a, smem, sh, tmem, c);
+            gemm_phase<PREC, 128, G3_INV_X>(a, smem, sh, tmem, c);
             if (!grid_sync(a.bar_count, a.bar_gen, a.flags, abort, a.bar_wait)) goto done;
-            gemm_phase<PREC, G4_INV_Y>(a, smem, sh, tmem, c);
+            gemm_phase<PREC, 128, G4_INV_Y>(a, smem, sh, tmem, c);
             if (!grid_sync(a.bar_count, a.bar_gen, a.flags, abort, a.bar_wait)) goto done;
             stencil_phase<T>(a, k, smem, sh, c);
             if (!grid_sync(a.bar_count, a.bar_gen, a.flags, abort, a.bar_wait)) goto done;
@@ -358,7 +368,7 @@ __global__ void __launch_bounds__(PT, 1) k_persistent(PersistArgs a) {
     }
 done:
     __syncthreads();
-    drain_after_abort<C::STAGES>(sh);
+    drain_after_abort(sh, tc_stages<PREC, 128>(a.tile_n));
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
@@ -383,11 +393,9 @@ size_t stencil_layout(int max_nl, PersistArgs* a) {
     return nbuf * slot + lap;
 }
 
-size_t persistent_smem_bytes(int precision, int max_nl, int large, PersistArgs* a) {
-    const size_t gemm = (precision == QG_DST_TF32 ? (size_t)TcCfg<QG_DST_TF32>::STAGES * tc_stage_bytes<QG_DST_TF32>()
-                                                  : (size_t)TcCfg<QG_DST_BF16X3>::STAGES * tc_stage_bytes<QG_DST_BF16X3>());
+size_t persistent_smem_bytes(int max_nl, int large, PersistArgs* a) {
     const size_t sten = large ? stencil_layout<st::TileL>(max_nl, a) : stencil_layout<st::TileS>(max_nl, a);
-    return std::max(gemm, sten) + 1024;
+    return std::max((size_t)TC_SMEM, sten) + 1024;
 }
 
 size_t stencil_mt_smem_bytes(int max_nl, int large, size_t* slot, size_t* lap_off, int* nbuf) {
@@ -418,22 +426,32 @@ cudaError_t launch_stencil_mt(const StencilArgs& sa, int n_st, int grid, int max
     return launch_k(k_stencil_mt<st::TileS>, grid, PT, smem, s, pdl, sa, n_st, slot, lap, nbuf);
 }
 
-template <int PREC>
-size_t gemm_mt_smem() {
-    return (size_t)TcCfg<PREC>::STAGES * tc_stage_bytes<PREC>() + 1024;
+template <int PREC, int ROW>
+size_t gemm_mt_smem(int bn) {
+    return (size_t)tc_stages<PREC, ROW>(bn) * tc_stage_bytes<PREC, ROW>(bn) + 1024;
 }
 
 cudaError_t launch_gemm_mt(const PersistArgs& a, int pass, int grid, int precision, cudaStream_t s, bool pdl) {
-#define QG_GMT(P)                                                                                                  \
-    switch (pass) {                                                                                                \
-        case G1_FWD_X: return launch_k(k_gemm_mt<P, G1_FWD_X>, grid, PT_GEMM, gemm_mt_smem<P>(), s, pdl, a);          \
-        case G2_FWD_Y: return launch_k(k_gemm_mt<P, G2_FWD_Y>, grid, PT_GEMM, gemm_mt_smem<P>(), s, pdl, a);          \
-        case G3_INV_X: return launch_k(k_gemm_mt<P, G3_INV_X>, grid, PT_GEMM, gemm_mt_smem<P>(), s, pdl, a);          \
-        case G4_INV_Y: return launch_k(k_gemm_mt<P, G4_INV_Y>, grid, PT_GEMM, gemm_mt_smem<P>(), s, pdl, a);          \
-        default: return cudaErrorInvalidValue;                                                                     \
+#define QG_GMT_PASS(P, R, PASS) \
+    case PASS: return launch_k(k_gemm_mt<P, R, PASS>, grid, PT_GEMM, gemm_mt_smem<P, R>(a.tile_n), s, pdl, a);
+#define QG_GMT(P, R)                 \
+    switch (pass) {                  \
+        QG_GMT_PASS(P, R, G1_FWD_X)  \
+        QG_GMT_PASS(P, R, G2_FWD_Y)  \
+        QG_GMT_PASS(P, R, G3_INV_X)  \
+        QG_GMT_PASS(P, R, G4_INV_Y)  \
+        default: return cudaErrorInvalidValue; \
     }
-    if (precision == QG_DST_TF32) { QG_GMT(QG_DST_TF32) }
-    if (precision == QG_DST_BF16X3) { QG_GMT(QG_DST_BF16X3) }
+    const bool wide = tc_row(a.tile_n) == 64;
+    if (precision == QG_DST_TF32) {
+        if (wide) QG_GMT(QG_DST_TF32, 64)
+        QG_GMT(QG_DST_TF32, 128)
+    }
+    if (precision == QG_DST_BF16X3) {
+        if (wide) QG_GMT(QG_DST_BF16X3, 64)
+        QG_GMT(QG_DST_BF16X3, 128)
+    }
+#undef QG_GMT_PASS
 #undef QG_GMT
     return cudaErrorInvalidValue;
 }
@@ -444,19 +462,27 @@ cudaError_t persistent_init() {
     if (!e) e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(B));
     QG_MTATTR(k_stencil_mt<st::TileS>, stencil_mt_smem_bytes(kMaxLayers, 0, nullptr, nullptr, nullptr))
     QG_MTATTR(k_stencil_mt<st::TileL>, stencil_mt_smem_bytes(kMaxLayers, 1, nullptr, nullptr, nullptr))
-    QG_MTATTR((k_gemm_mt<QG_DST_TF32, G1_FWD_X>), gemm_mt_smem<QG_DST_TF32>())
-    QG_MTATTR((k_gemm_mt<QG_DST_TF32, G2_FWD_Y>), gemm_mt_smem<QG_DST_TF32>())
-    QG_MTATTR((k_gemm_mt<QG_DST_TF32, G3_INV_X>), gemm_mt_smem<QG_DST_TF32>())
-    QG_MTATTR((k_gemm_mt<QG_DST_TF32, G4_INV_Y>), gemm_mt_smem<QG_DST_TF32>())
-    QG_MTATTR((k_gemm_mt<QG_DST_BF16X3, G1_FWD_X>), gemm_mt_smem<QG_DST_BF16X3>())
-    QG_MTATTR((k_gemm_mt<QG_DST_BF16X3, G2_FWD_Y>), gemm_mt_smem<QG_DST_BF16X3>())
-    QG_MTATTR((k_gemm_mt<QG_DST_BF16X3, G3_INV_X>), gemm_mt_smem<QG_DST_BF16X3>())
-    QG_MTATTR((k_gemm_mt<QG_DST_BF16X3, G4_INV_Y>), gemm_mt_smem<QG_DST_BF16X3>())
+    QG_MTATTR((k_gemm_mt<QG_DST_TF32, 128, G1_FWD_X>), TC_SMEM + 1024)
+    QG_MTATTR((k_gemm_mt<QG_DST_TF32, 64, G1_FWD_X>), TC_SMEM + 1024)
+    QG_MTATTR((k_gemm_mt<QG_DST_TF32, 128, G2_FWD_Y>), TC_SMEM + 1024)
+    QG_MTATTR((k_gemm_mt<QG_DST_TF32, 64, G2_FWD_Y>), TC_SMEM + 1024)
+    QG_MTATTR((k_gemm_mt<QG_DST_TF32, 128, G3_INV_X>), TC_SMEM + 1024)
+    QG_MTATTR((k_gemm_mt<QG_DST_TF32, 64, G3_INV_X>), TC_SMEM + 1024)
+    QG_MTATTR((k_gemm_mt<QG_DST_TF32, 128, G4_INV_Y>), TC_SMEM + 1024)
+    QG_MTATTR((k_gemm_mt<QG_DST_TF32, 64, G4_INV_Y>), TC_SMEM + 1024)
+    QG_MTATTR((k_gemm_mt<QG_DST_BF16X3, 128, G1_FWD_X>), TC_SMEM + 1024)
+    QG_MTATTR((k_gemm_mt<QG_DST_BF16X3, 64, G1_FWD_X>), TC_SMEM + 1024)
+    QG_MTATTR((k_gemm_mt<QG_DST_BF16X3, 128, G2_FWD_Y>), TC_SMEM + 1024)
+    QG_MTATTR((k_gemm_mt<QG_DST_BF16X3, 64, G2_FWD_Y>), TC_SMEM + 1024)
+    QG_MTATTR((k_gemm_mt<QG_DST_BF16X3, 128, G3_INV_X>), TC_SMEM + 1024)
+    QG_MTATTR((k_gemm_mt<QG_DST_BF16X3, 64, G3_INV_X>), TC_SMEM + 1024)
+    QG_MTATTR((k_gemm_mt<QG_DST_BF16X3, 128, G4_INV_Y>), TC_SMEM + 1024)
+    QG_MTATTR((k_gemm_mt<QG_DST_BF16X3, 64, G4_INV_Y>), TC_SMEM + 1024)
 #undef QG_MTATTR
 #define QG_PATTR(P, T, L)                                                                                      \
     if (!e)                                                                                                    \
         e = cudaFuncSetAttribute(k_persistent<P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,              \
-                                 (int)persistent_smem_bytes(P, kMaxLayers, L, nullptr));
+                                 (int)persistent_smem_bytes(kMaxLayers, L, nullptr));
     QG_PATTR(QG_DST_TF32, st::TileS, 0)
     QG_PATTR(QG_DST_TF32, st::TileL, 1)
     QG_PATTR(QG_DST_BF16X3, st::TileS, 0)
@@ -469,7 +495,7 @@ cudaError_t launch_persistent(const PersistArgs& a, int grid, int precision, cud
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(PT);
-    cfg.dynamicSmemBytes = persistent_smem_bytes(precision, a.max_nl, a.st_large, nullptr);
+    cfg.dynamicSmemBytes = persistent_smem_bytes(a.max_nl, a.st_large, nullptr);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;  // all CTAs co-resident: the grid barrier needs it

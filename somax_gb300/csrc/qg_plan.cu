@@ -18,7 +18,6 @@
 
 namespace qg {
 cudaError_t gemm_tc_init();
-int gemm_tc_tile_n(int precision);
 }  // namespace qg
 
 using namespace qg;
@@ -228,6 +227,10 @@ struct StepGraph {
     int scheme = -1;
 };
 
+// Tensor-core output tile widths: a caller may force the first kForcedBN, the autotuner takes any.
+constexpr int kNumBN = 8, kForcedBN = 5;
+constexpr int kGemmBN[kNumBN] = {144, 80, 48, 32, 16, 176, 208, 256};
+
 // The captured launch sequence of one qg_step_vjp call and the arguments it was captured with
 // (replayed while they repeat).
 struct VjpGraph {
@@ -252,12 +255,13 @@ struct qg_plan {
     GemmTile* gx_tiles = nullptr;  // passes with A in x-row planes (G1, G4)
     GemmTile* gy_tiles = nullptr;  // passes with A in y-row planes (G2, G3)
     int n_gx = 0, n_gy = 0;
-    // tensor-core tile lists for each candidate output tile width (kGemmBN); the autotuner
-    // keeps the fastest (wide tiles for large members, narrow ones spread small members)
-    GemmTile* gx_v[5] = {};
-    GemmTile* gy_v[5] = {};
-    int n_gx_v[5] = {}, n_gy_v[5] = {};
-    int n_bn = 1, bn_sel = 0;
+    // tensor-core tile lists and TMA descriptors for each candidate output tile width (kGemmBN;
+    // null: not a candidate); the autotuner keeps the fastest
+    GemmTile* gx_v[kNumBN] = {};
+    GemmTile* gy_v[kNumBN] = {};
+    int n_gx_v[kNumBN] = {}, n_gy_v[kNumBN] = {};
+    void* tc_maps_v[kNumBN] = {};
+    int bn_sel = 0;
     int simt_sel = 0;  // tile shape of the FP32 passes
     // FP32 row engine (qg_rows.cu): the constant part of its launches' arguments, whether the
     // members allow it, whether the plan runs it, and the autotuner's time
@@ -265,7 +269,7 @@ struct qg_plan {
     ColsArgs rc{};
     bool rw_ok = false, rw_on = false;
     float tune_rows_ms = -1.f;
-    float tune_gemm_ms[5] = {-1.f, -1.f, -1.f, -1.f, -1.f};
+    float tune_gemm_ms[kNumBN];
     // cluster-resident stepping (qg_cluster.cu): CTAs per member's cluster (0: not possible),
     // its dynamic shared memory, the members' layer count, whether qg_step uses it, and the
     // autotuner's times of four SSP-RK3 steps (multi-launch, cluster)
@@ -291,7 +295,6 @@ struct qg_plan {
     void* stats_acc = nullptr;  // qg_state_stats accumulators (32 bytes)
     double* vjp_acc = nullptr;  // parameter cotangents of qg_rhs_vjp (QG_NPARAMS per member)
     int op_fmt = FMT_F32;
-    void* tc_maps = nullptr;  // TMA descriptors of the tensor-core GEMMs
     void* st_maps = nullptr;  // TMA descriptors of the stencil halo boxes
     unsigned* bar = nullptr;  // grid barrier words of the persistent kernel (count, generation)
     int n_sm = 0;
@@ -398,7 +401,7 @@ GemmArgs gemm_args(qg_plan* p, int pass, const void* A, void* C, int a_fmt, int 
     g.a_fmt = a_fmt;
     g.c_fmt = c_fmt;
     g.accumulate = acc;
-    g.tc_maps = p->tc_maps;
+    g.tc_maps = p->pa.tc_maps;
     g.flags = p->flags;
     return g;
 }
@@ -569,8 +572,6 @@ StencilArgs stencil_args(qg_plan* p, const float* params) {
 }
 
 constexpr int kSweepRows[3] = {16, 32, 64};  // strip heights of sweep list v: kSweepRows[v % 3]
-constexpr int kNumBN = 5;
-constexpr int kGemmBN[kNumBN] = {144, 80, 48, 32, 16};  // tensor-core output tile widths the autotuner tries
 
 // The multi-launch path's stencil launch: the column sweep if selected, else the tiles.
 cudaError_t launch_stencil(qg_plan* p, StencilArgs a, cudaStream_t s, bool pdl) {
@@ -787,7 +788,7 @@ void select_tile(qg_plan* p, int large) {
     a.n_st = p->n_st;
     a.st_maps = p->st_maps;
     a.st_large = large;
-    if (p->opts.dst_precision != QG_DST_FP32) persistent_smem_bytes(p->opts.dst_precision, p->max_nl, large, &a);
+    if (p->opts.dst_precision != QG_DST_FP32) persistent_smem_bytes(p->max_nl, large, &a);
 }
 
 // Make tensor-core tile width kGemmBN[v] the active one (tile lists, persistent arguments).
@@ -803,9 +804,28 @@ void select_gemm(qg_plan* p, int v) {
     a.n_gx = p->n_gx;
     a.n_gy = p->n_gy;
     a.tile_n = kGemmBN[v];
+    a.tc_maps = p->tc_maps_v[v];
 }
 
-// Autotuner: time the four DST passes with each tensor-core tile width (zero planes) and keep
+// Cycles the busiest CTA of a pass needs for its tiles of width bn, from what bounds them: a k-block
+// is loaded at about 45 bytes a cycle or multiplied at 4096 products a cycle, a tile drained in 1500.
+// Orders the widths before any is timed; the timing decides.
+double gemm_estimate(const std::vector<GemmTile>& list, int n_sm, const std::vector<int>& kdim, int precision, int bn) {
+    const bool bf = precision == QG_DST_BF16X3;
+    const int row = bn > 144 ? 64 : 128, bk = bf ? row / 2 : row / 4;
+    const double block = std::max((bf ? 2 : 1) * (128 + bn) * row / 45.0, 128.0 * bn * bk * (bf ? 3 : 2) / 4096.0);
+    const int G = std::max(1, std::min((int)list.size(), n_sm));
+    double worst = 0.0;
+    for (int b = 0; b < G; ++b) {
+        double c = 0.0;
+        for (size_t t = b; t < list.size(); t += G)
+            if (list[t].member >= 0) c += (kdim[list[t].member] + bk - 1) / bk * block + 1500.0;
+        worst = std::max(worst, c);
+    }
+    return worst;
+}
+
+// Autotuner: time the four DST passes with each candidate tile width (zero planes) and keep
 // the fastest.
 cudaError_t autotune_gemm(qg_plan* p) {
     cudaStream_t s = p->cap;
@@ -813,8 +833,9 @@ cudaError_t autotune_gemm(qg_plan* p) {
     cudaError_t e = cudaEventCreate(&e0);
     if (!e) e = cudaEventCreate(&e1);
     if (e) return e;
-    int best = 0;
-    for (int v = 0; v < p->n_bn && !e; ++v) {
+    int best = -1;
+    for (int v = 0; v < kNumBN && !e; ++v) {
+        if (!p->tc_maps_v[v]) continue;
         select_gemm(p, v);
         float ms = 0.f;
         e = run_dst_solve(p, s);
@@ -824,11 +845,11 @@ cudaError_t autotune_gemm(qg_plan* p) {
         if (!e) e = cudaEventSynchronize(e1);
         if (!e) e = cudaEventElapsedTime(&ms, e0, e1);
         p->tune_gemm_ms[v] = ms / 3.f;
-        if (!e && p->tune_gemm_ms[v] < p->tune_gemm_ms[best]) best = v;
+        if (!e && (best < 0 || p->tune_gemm_ms[v] < p->tune_gemm_ms[best])) best = v;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    if (!e) select_gemm(p, best);
+    if (!e && best >= 0) select_gemm(p, best);
     return e;
 }
 
@@ -906,7 +927,7 @@ cudaError_t autotune_stencil(qg_plan* p) {
 
 namespace qg {
 cudaError_t tmap_encode(void* map, int bf16, int rank, const void* base, const uint64_t* dims,
-                        const uint64_t* strides_bytes, const uint32_t* box, int swizzle128) {
+                        const uint64_t* strides_bytes, const uint32_t* box, int swizzle) {
     if (!g_encode || rank < 1 || rank > 5) return cudaErrorInvalidValue;
     const int es = bf16 ? 2 : 4;
     if (((uintptr_t)base & 15) || (box[0] * es) % 16) return cudaErrorInvalidValue;
@@ -925,7 +946,9 @@ cudaError_t tmap_encode(void* map, int bf16, int rank, const void* base, const u
     CUresult r = g_encode(static_cast<CUtensorMap*>(map),
                           bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, rank,
                           const_cast<void*>(base), d, st, b, e, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                          swizzle == 128  ? CU_TENSOR_MAP_SWIZZLE_128B
+                          : swizzle == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                          : CU_TENSOR_MAP_SWIZZLE_NONE,
                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
@@ -957,7 +980,7 @@ int qg_plan_create(const qg_member_desc* members, int n_members, const qg_option
     if (o.refine_sweeps < 0 || o.refine_sweeps > 1) return QG_ERR_ARG;
     if (o.cluster < 0 || o.cluster > 2) return QG_ERR_ARG;
     if (o.stencil < 0 || o.stencil > QG_STENCIL_VARIANTS) return QG_ERR_ARG;
-    if (o.gemm_tile != 0 && std::find(kGemmBN, kGemmBN + kNumBN, o.gemm_tile) == kGemmBN + kNumBN)
+    if (o.gemm_tile != 0 && std::find(kGemmBN, kGemmBN + kForcedBN, o.gemm_tile) == kGemmBN + kForcedBN)
         return QG_ERR_ARG;
     for (int i = 0; i < n_members; ++i) {
         const int v = validate_member(members[i]);
@@ -965,6 +988,7 @@ int qg_plan_create(const qg_member_desc* members, int n_members, const qg_option
     }
     qg_plan* p = new (std::nothrow) qg_plan();
     if (!p) return QG_ERR_CUDA;
+    std::fill(p->tune_gemm_ms, p->tune_gemm_ms + kNumBN, -1.f);
     p->n_members = n_members;
     p->opts = o;
     p->desc.assign(members, members + n_members);
@@ -1015,6 +1039,7 @@ int qg_plan_create(const qg_member_desc* members, int n_members, const qg_option
         p->simt_sel = simt_shape(tiles, std::max(p->n_sm, 1));
     }
     const int n_bn = tc ? kNumBN : 1;
+    bool candidate[kNumBN] = {};  // tile widths the plan keeps lists and descriptors of
     std::vector<GemmTile> gxv[kNumBN], gyv[kNumBN];
     std::map<long long, std::pair<float*, uint16_t*>> dst_cache;  // (size, pitch) -> device DST-I matrix
     // the row engine: no refinement, land or forced variant, members alike in layers and grid; it
@@ -1193,7 +1218,6 @@ int qg_plan_create(const qg_member_desc* members, int n_members, const qg_option
         e = upload(p, &p->md, mv);
     }
     if (e == cudaSuccess) {
-        p->n_bn = n_bn;
         for (int v = 0; v < 2 && !e; ++v) {
             p->n_st_v[v] = (int)st_v[v].size();
             e = upload(p, &p->st_tiles_v[v], st_v[v]);
@@ -1233,17 +1257,32 @@ int qg_plan_create(const qg_member_desc* members, int n_members, const qg_option
                 gxv[v] = schedule_tiles(gxv[v], p->n_sm, kx);
                 gyv[v] = schedule_tiles(gyv[v], p->n_sm, ky);
             }
+            // the widths to time: the forced one, the default without autotuning, else the four
+            // the estimate puts first, as far as they are within 40% of the best
+            // (the persistent kernel takes 128-byte rows only)
+            const bool persist = o.persistent && o.refine_sweeps == 0;
+            std::vector<std::pair<double, int>> est;
+            for (int v = 0; v < n_bn; ++v)
+                if (o.gemm_tile ? kGemmBN[v] == o.gemm_tile : (o.autotune && (v < kForcedBN || !persist)) || v == 0)
+                    est.push_back({gemm_estimate(gxv[v], p->n_sm, kx, o.dst_precision, kGemmBN[v]) +
+                                       gemm_estimate(gyv[v], p->n_sm, ky, o.dst_precision, kGemmBN[v]),
+                                   v});
+            std::sort(est.begin(), est.end());
+            for (size_t k = 0; k < est.size() && k < 4 && est[k].first <= 1.4 * est[0].first; ++k)
+                candidate[est[k].second] = true;
         }
         for (int v = 0; v < n_bn && !e; ++v) {
+            if (tc && !candidate[v]) continue;
             p->n_gx_v[v] = (int)gxv[v].size();
             p->n_gy_v[v] = (int)gyv[v].size();
             if (!(e = upload(p, &p->gx_v[v], gxv[v]))) e = upload(p, &p->gy_v[v], gyv[v]);
         }
         if (!e) {
-            p->gx_tiles = p->gx_v[0];
-            p->gy_tiles = p->gy_v[0];
-            p->n_gx = p->n_gx_v[0];
-            p->n_gy = p->n_gy_v[0];
+            while (p->bn_sel + 1 < n_bn && !candidate[p->bn_sel]) ++p->bn_sel;
+            p->gx_tiles = p->gx_v[p->bn_sel];
+            p->gy_tiles = p->gy_v[p->bn_sel];
+            p->n_gx = p->n_gx_v[p->bn_sel];
+            p->n_gy = p->n_gy_v[p->bn_sel];
         }
     }
     if (e == cudaSuccess) {
@@ -1260,15 +1299,18 @@ int qg_plan_create(const qg_member_desc* members, int n_members, const qg_option
         if (!e) e = dalloc(p, &p->K, (size_t)6 * p->state_size * sizeof(float));  // Tsit5: 6 stages
     }
     if (e == cudaSuccess && tc) {
-        // one set of TMA descriptors per (member, pass); the planes never move
+        // one set of TMA descriptors per (member, pass) and tile width; the planes never move
         std::vector<uint8_t> maps((size_t)n_members * 4 * kTcMapsBytes);
         const void* in_plane[4] = {p->XA, p->YA, p->XB, p->YB};
         const int64_t in_elems[4] = {p->xplane, p->yplane, p->xplane, p->yplane};
-        for (int i = 0; i < n_members && !e; ++i)
-            for (int pass = 0; pass < 4 && !e; ++pass)
-                e = gemm_tc_encode(p->mh[i], pass, in_plane[pass], in_elems[pass], o.dst_precision,
-                                   maps.data() + ((size_t)i * 4 + pass) * kTcMapsBytes);
-        if (!e) e = upload(p, (uint8_t**)&p->tc_maps, maps);
+        for (int v = 0; v < kNumBN && !e; ++v) {
+            if (!candidate[v]) continue;
+            for (int i = 0; i < n_members && !e; ++i)
+                for (int pass = 0; pass < 4 && !e; ++pass)
+                    e = gemm_tc_encode(p->mh[i], pass, in_plane[pass], in_elems[pass], o.dst_precision, kGemmBN[v],
+                                       maps.data() + ((size_t)i * 4 + pass) * kTcMapsBytes);
+            if (!e) e = upload(p, (uint8_t**)&p->tc_maps_v[v], maps);
+        }
     }
     if (e == cudaSuccess) {
         // TMA descriptors of the stencil's halo boxes: the three stage planes and psi_hat
@@ -1288,9 +1330,9 @@ int qg_plan_create(const qg_member_desc* members, int n_members, const qg_option
         a.gy = p->gy_tiles;
         a.n_gx = p->n_gx;
         a.n_gy = p->n_gy;
-        a.tile_n = kGemmBN[0];
+        a.tile_n = kGemmBN[p->bn_sel];
         a.max_nl = p->max_nl;
-        a.tc_maps = p->tc_maps;
+        a.tc_maps = p->tc_maps_v[p->bn_sel];
         a.XA = p->XA;
         a.YA = p->YA;
         a.YB = p->YB;
@@ -1317,9 +1359,6 @@ int qg_plan_create(const qg_member_desc* members, int n_members, const qg_option
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->fork_ev, cudaEventDisableTiming);
         // a forced choice (qg_options.gemm_tile / .stencil) skips that half of the autotuner
         if (!e && o.autotune && tc && !o.gemm_tile) e = autotune_gemm(p);
-        if (!e && tc && o.gemm_tile)
-            for (int v = 0; v < kNumBN; ++v)
-                if (kGemmBN[v] == o.gemm_tile) select_gemm(p, v);
         if (!e && o.autotune && !o.stencil) e = autotune_stencil(p);
         if (!e && o.stencil > 0) {
             // a forced variant (tests, benchmarks of one variant)

@@ -2,8 +2,14 @@
 // (qg_gemm_tc.cu) and the persistent step kernel (qg_persistent.cu).
 //
 // C = A * S with A rows (layer, r) K-major and S symmetric (so its rows are the K-major B
-// operand).  Operands are 128-byte rows in 128-byte-swizzled shared memory (the layout TMA
-// writes with SWIZZLE_128B); the FP32 accumulator is a 128-lane x BN-column TMEM block.
+// operand).  Operands are ROW-byte rows in ROW-byte-swizzled shared memory (the layout TMA writes
+// with SWIZZLE_128B or SWIZZLE_64B); the FP32 accumulator is a 128-lane x BN-column TMEM block.
+//
+// Bound: the latency of the ring of k-blocks and what a CTA takes from L2 (about 45 bytes a cycle), and
+// how many whole waves a pass's tiles make.  Rows of 128 bytes up to 144 columns; wider tiles take
+// 64-byte rows, of which five stages fit where two of 128 bytes would (all widths in 64-byte rows made
+// the 256-member ensemble's steps 7% slower).  A tile stages only the S rows of its own width (a
+// 16-wide tile used to stage 144).
 #pragma once
 
 #include <cuda.h>
@@ -15,14 +21,18 @@
 namespace qg {
 
 constexpr int TC_BM = 128;
-// Largest output tile width (N): 144 = 9 x 16 so that the N = n + 2 sizes of the DST (66,
-// 130, 258, 514) need one, one, two and four tiles; a plan may cut narrower tiles (more
-// CTAs for small members), and the last tile of a member runs its MMAs at the width it needs
-// (a multiple of 16), so little of the tensor work is padding.  The S operand's TMA box is
-// always TC_BN rows.
-constexpr int TC_BN = 144;
+// Largest output tile width (N).  A plan cuts its passes into tiles of one width: 144 = 9 x 16 for
+// the N = n + 2 sizes of the DST (66, 130, 258, 514: one, one, two and four tiles), narrower ones to
+// spread small members over more CTAs, wider ones where they save a wave (1026 columns of three
+// layers: 150 tiles of 176 for 152 CTAs, where 144 made 200); the last tile of a member runs its
+// MMAs at the width it needs (a multiple of 16), so little of the tensor work is padding.
+constexpr int TC_BN = 256;
 constexpr int TC_TMEM_BUF = 256;   // TMEM column stride of the two accumulators
 constexpr int TC_TMEM_COLS = 512;  // allocation (power of two >= 2 buffers)
+// Bytes of an operand row of one k-block for tiles of bn columns.
+__host__ __device__ constexpr int tc_row(int bn) { return bn > 144 ? 64 : 128; }
+constexpr int TC_MAX_STAGES = 10;
+constexpr int TC_SMEM = 216 * 1024;  // shared memory of the k-block ring
 // Width of output tile nt of a pass with Nn columns cut into tiles of bn (<= TC_BN) columns.
 __host__ __device__ constexpr int tc_tile_width(int Nn, int nt, int bn) {
     return (Nn - nt * bn >= bn) ? bn : ((Nn - nt * bn + 15) / 16) * 16;
@@ -30,60 +40,62 @@ __host__ __device__ constexpr int tc_tile_width(int Nn, int nt, int bn) {
 
 struct TcMaps {
     CUtensorMap a[2];  // A hi (or f32), A lo
-    CUtensorMap b[2];  // S hi (or f32), S lo
+    CUtensorMap b[2];  // S hi (or f32), S lo: boxes of one tile width
 };
 static_assert(sizeof(TcMaps) == kTcMapsBytes, "TcMaps size");
 
-template <int PREC>
+template <int PREC, int ROW>
 struct TcCfg;
-template <>
-struct TcCfg<QG_DST_TF32> {
-    static constexpr int BK = 32;  // 32 fp32 = 128-byte rows
-    static constexpr int STAGES = 4;
+template <int ROW>
+struct TcCfg<QG_DST_TF32, ROW> {
+    static constexpr int BK = ROW / 4;
     static constexpr int ESIZE = 4;
     static constexpr int NA = 1, NB = 1;  // operand planes
     static constexpr int UMMA_K = 8;      // 32 bytes per MMA along K
     static constexpr uint32_t FMT = 2;    // tf32
 };
-template <>
-struct TcCfg<QG_DST_BF16X3> {
-    static constexpr int BK = 64;  // 64 bf16 = 128-byte rows
-    static constexpr int STAGES = 3;
+template <int ROW>
+struct TcCfg<QG_DST_BF16X3, ROW> {
+    static constexpr int BK = ROW / 2;
     static constexpr int ESIZE = 2;
     static constexpr int NA = 2, NB = 2;  // hi, lo
     static constexpr int UMMA_K = 16;
     static constexpr uint32_t FMT = 1;    // bf16
 };
 
-template <int PREC>
-__host__ __device__ constexpr int tc_tile_a_bytes() { return TC_BM * TcCfg<PREC>::BK * TcCfg<PREC>::ESIZE; }
-template <int PREC>
-__host__ __device__ constexpr int tc_tile_b_bytes() { return TC_BN * TcCfg<PREC>::BK * TcCfg<PREC>::ESIZE; }
-template <int PREC>
-__host__ __device__ constexpr int tc_stage_bytes() {
-    return TcCfg<PREC>::NA * tc_tile_a_bytes<PREC>() + TcCfg<PREC>::NB * tc_tile_b_bytes<PREC>();
+// One k-block of a tile of bn columns (a multiple of 16: every plane starts on a 1024-byte boundary),
+// and the stages of them that fit.
+template <int PREC, int ROW>
+__host__ __device__ constexpr int tc_stage_bytes(int bn) {
+    return TcCfg<PREC, ROW>::NA * TC_BM * ROW + TcCfg<PREC, ROW>::NB * bn * ROW;
+}
+template <int PREC, int ROW>
+__host__ __device__ constexpr int tc_stages(int bn) {
+    const int n = TC_SMEM / tc_stage_bytes<PREC, ROW>(bn);
+    return n < TC_MAX_STAGES ? n : TC_MAX_STAGES;
 }
 
 // Instruction descriptor: D f32, A/B format FMT, both K-major, N = n (a multiple of 16 up to
 // TC_BN), M = TC_BM.
 template <int PREC>
 __device__ __forceinline__ uint32_t tc_idesc(int n) {
-    return (1u << 4) | (TcCfg<PREC>::FMT << 7) | (TcCfg<PREC>::FMT << 10) | ((uint32_t)(n >> 3) << 17) |
+    return (1u << 4) | (TcCfg<PREC, 128>::FMT << 7) | (TcCfg<PREC, 128>::FMT << 10) | ((uint32_t)(n >> 3) << 17) |
            ((uint32_t)(TC_BM >> 4) << 24);
 }
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, 8-row groups 1024
-// bytes apart (SBO), descriptor version 1.
+// Shared-memory matrix descriptor: K-major operand, ROW-byte swizzle, groups of 8 rows one after the
+// other (SBO), descriptor version 1.
+template <int ROW>
 __device__ __forceinline__ uint64_t tc_sdesc(uint32_t saddr) {
     uint64_t d = 0;
     d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
     d |= (uint64_t)1 << 16;            // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;  // stride byte offset
+    d |= (uint64_t)(8 * ROW >> 4) << 32;  // stride byte offset
     d |= (uint64_t)1 << 46;            // version
-    d |= (uint64_t)2 << 61;            // SWIZZLE_128B
+    d |= (uint64_t)(ROW == 128 ? 2 : 4) << 61;  // SWIZZLE_128B, SWIZZLE_64B
     return d;
 }
 
@@ -187,20 +199,20 @@ __device__ __forceinline__ float tc_rowterm(const TcTile& T, int quarter, int la
 // Issue the MMAs of one k-block (operands at shared addresses sa / sb) into tmem_d: `ksteps`
 // UMMA_K-wide steps (the last k-block of a member stops at its K; the zero fill beyond it
 // contributes nothing) at output width n.
-template <int PREC>
-__device__ __forceinline__ void tc_mma_kblock(uint32_t tmem_d, uint32_t sa, uint32_t sb, bool first, int ksteps,
-                                              int n) {
-    using C = TcCfg<PREC>;
+template <int PREC, int ROW>
+__device__ __forceinline__ void tc_mma_kblock(uint32_t tmem_d, uint32_t sa, uint32_t sb, uint32_t b_bytes, bool first,
+                                              int ksteps, int n) {
+    using C = TcCfg<PREC, ROW>;
     const uint32_t idesc = tc_idesc<PREC>(n);
 #pragma unroll
     for (int k = 0; k < C::BK / C::UMMA_K; ++k) {
         if (k >= ksteps) break;
         const uint32_t koff = k * C::UMMA_K * C::ESIZE;  // 32 bytes per step
-        const uint64_t a0 = tc_sdesc(sa + koff), b0 = tc_sdesc(sb + koff);
+        const uint64_t a0 = tc_sdesc<ROW>(sa + koff), b0 = tc_sdesc<ROW>(sb + koff);
         tc_mma<C::FMT>(tmem_d, a0, b0, idesc, (!first || k > 0) ? 1u : 0u);
         if constexpr (C::NA == 2) {
-            const uint64_t a1 = tc_sdesc(sa + tc_tile_a_bytes<PREC>() + koff);
-            const uint64_t b1 = tc_sdesc(sb + tc_tile_b_bytes<PREC>() + koff);
+            const uint64_t a1 = tc_sdesc<ROW>(sa + TC_BM * ROW + koff);
+            const uint64_t b1 = tc_sdesc<ROW>(sb + b_bytes + koff);
             tc_mma<C::FMT>(tmem_d, a0, b1, idesc, 1u);  // Ahi * Slo
             tc_mma<C::FMT>(tmem_d, a1, b0, idesc, 1u);  // Alo * Shi
         }
@@ -238,7 +250,7 @@ __device__ __forceinline__ void tc_epilogue(const TcTile& T, void* Cv, int c_fmt
     float* Cf = static_cast<float*>(Cv) + g.cbase;
     __nv_bfloat16* Cb = static_cast<__nv_bfloat16*>(Cv) + g.cbase;
     const int64_t obase = (int64_t)l * Nn * ldo + r;
-    for (int c = c0; c < (TC_BN + 31) / 32; c += cstep) {
+    for (int c = c0; c * 32 < T.width; c += cstep) {
         const int nb = n0 + c * 32;
         if (!valid || nb >= nend) break;  // warp-uniform (and the same for every epilogue warp)
         float eyl = 1.f;
@@ -259,20 +271,26 @@ __device__ __forceinline__ void tc_epilogue(const TcTile& T, void* Cv, int c_fmt
         const int64_t o0 = obase + (int64_t)nb * ldo;
         if (c_fmt == FMT_F32) {
             float* q = Cf + o0;
+            if (PASS == G4_INV_Y && accumulate) {
+                // loads ahead of the stores, sixteen at a time: in turn they would cost a trip to L2
+                // each (15 us a pass at 1024 x 1024 x 3)
+#pragma unroll
+                for (int h = 0; h < 32; h += 16) {
+                    float old[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) old[j] = h + j < ncol ? q[(int64_t)(h + j) * ldo] : 0.f;
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[h + j] = __float_as_uint(__uint_as_float(v[h + j]) + old[j]);
+                }
+            }
             if (ncol == 32) {
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    float x = __uint_as_float(v[j]);
-                    if (PASS == G4_INV_Y && accumulate) x += q[(int64_t)j * ldo];
-                    q[(int64_t)j * ldo] = x;
-                }
+                for (int j = 0; j < 32; ++j) q[(int64_t)j * ldo] = __uint_as_float(v[j]);
             } else {
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
                     if (j >= ncol) break;
-                    float x = __uint_as_float(v[j]);
-                    if (PASS == G4_INV_Y && accumulate) x += q[(int64_t)j * ldo];
-                    q[(int64_t)j * ldo] = x;
+                    q[(int64_t)j * ldo] = __uint_as_float(v[j]);
                 }
             }
         } else {

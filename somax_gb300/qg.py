@@ -443,12 +443,12 @@ class Plan:
         ms = (C.c_float * n)()
         check(self._L.qg_plan_tuning(self._h, C.byref(v), ms, n), "qg_plan_tuning")
         bn = C.c_int()
-        gms = (C.c_float * 5)()
-        check(self._L.qg_plan_gemm_tuning(self._h, C.byref(bn), gms, 5), "qg_plan_gemm_tuning")
+        gms = (C.c_float * 8)()
+        check(self._L.qg_plan_gemm_tuning(self._h, C.byref(bn), gms, len(gms)), "qg_plan_gemm_tuning")
         return {"stencil": self.STENCIL_VARIANTS[v.value],
                 "ms": {name: round(float(t), 5) for name, t in zip(self.STENCIL_VARIANTS, ms)},
                 "gemm_tile_n": bn.value,
-                "gemm_ms": {w: round(float(t), 5) for w, t in zip((144, 80, 48, 32, 16), gms)}}
+                "gemm_ms": {w: round(float(t), 5) for w, t in zip((144, 80, 48, 32, 16, 176, 208, 256), gms)}}
 
     def engine(self) -> dict:
         """The stepping engine of ``step`` (Heun / SSP-RK3): the cluster size of the cluster-
