@@ -214,71 +214,71 @@ __global__ void __launch_bounds__(NT) k_vjp_tau(const MemberDev* __restrict__ me
 // Right-hand side of the adjoint solve in the GEMM operand format (plus its FP32 copy for the
 // refinement residual).  From the FP32 modal plane `rhs` when `psi_bar` is null, else
 // Cm2l^T Z psi_bar of a caller-packed layer cotangent (the VJP of the inversion).
-__global__ void __launch_bounds__(NT) k_vjp_operand(const MemberDev* members, const StencilTile* tiles, int TX, int TY,
-                                                    int parts, const float* rhs, const float* psi_bar, void* xa,
-                                                    int xa_fmt, float* xq, int64_t xplane) {
+__global__ void __launch_bounds__(NT, 4) k_vjp_operand(const MemberDev* members, const StencilTile* tiles, int parts,
+                                                    const float* rhs, const float* psi_bar, void* xa, int xa_fmt,
+                                                    float* xq, int64_t xplane) {
     __shared__ MemberDev M;
     const StencilTile t = tiles[blockIdx.x / (unsigned)parts];
     st::load_member(&M, members + t.member);
     __syncthreads();
     pdl_wait();
     pdl_launch_dependents();
+    const st::CellGeom G(M);
     st::with_layers(M.nl, [&](auto n) {
         constexpr int NL = decltype(n)::value;
+        const st::Mix<NL, true> C(M.Cm2l);
+        const bool keep_ring = M.barotropic;
         st::walk_cells<NL, NL <= 4 ? 4 : 2>(
-            M, t, TX, TY, parts,
+            G, t, parts,
             [&](int j, int i, float(&x)[NL]) {
+                const int64_t c = G.c(j, i), o = G.x(j, i);
 #pragma unroll
-                for (int l = 0; l < NL; ++l) x[l] = psi_bar ? psi_bar[cidx(M, l, j, i)] : rhs[xidx(M, l, j, i)];
+                for (int l = 0; l < NL; ++l) x[l] = psi_bar ? psi_bar[c + l * G.lc] : rhs[o + l * G.lx];
             },
             [&](int j, int i, float(&x)[NL]) {
-                const bool zero = (!M.barotropic && on_ring(j, i, M.Ny, M.Nx)) || is_land(M.mask, M.Ny, M.Nx, j, i);
+                const bool zero = (!keep_ring && G.ring(j, i)) || G.land(j, i);
+                const int64_t o = G.x(j, i);
 #pragma unroll
                 for (int m = 0; m < NL; ++m) {
-                    const int64_t o = xidx(M, m, j, i);
-                    float v = 0.f;
-                    if (!psi_bar)
-                        v = x[m];
-                    else if (!zero)
-#pragma unroll
-                        for (int l = 0; l < NL; ++l) v = fmaf(M.Cm2l[l * kMaxLayers + m], x[l], v);
-                    st::store_plane(xa, xa_fmt, xplane, o, v);
-                    if (xq) xq[o] = v;
+                    const float v = !psi_bar ? x[m] : zero ? 0.f : C.row(m, x);
+                    st::store_plane(xa, xa_fmt, xplane, o + m * G.lx, v);
+                    if (xq) xq[o + m * G.lx] = v;
                 }
             });
     });
 }
 
 // q_bar = B (direct + Cl2m^T x_bar) in caller packing, x_bar the adjoint solve's output.
-__global__ void __launch_bounds__(NT) k_vjp_finish(const MemberDev* members, const StencilTile* tiles, int TX, int TY,
-                                                   int parts, const float* direct, const float* xbar, int apply_bc,
-                                                   float* qbar) {
+__global__ void __launch_bounds__(NT, 4) k_vjp_finish(const MemberDev* members, const StencilTile* tiles, int parts,
+                                                   const float* direct, const float* xbar, int apply_bc, float* qbar) {
     __shared__ MemberDev M;
     const StencilTile t = tiles[blockIdx.x / (unsigned)parts];
     st::load_member(&M, members + t.member);
     __syncthreads();
     pdl_wait();
     pdl_launch_dependents();
+    const st::CellGeom G(M);
     st::with_layers(M.nl, [&](auto n) {
         constexpr int NL = decltype(n)::value;
-        st::walk_cells<2 * NL, NL <= 2 ? 4 : 2>(
-            M, t, TX, TY, parts,
+        const st::Mix<NL, true> C(M.Cl2m);
+        st::walk_cells<2 * NL, NL <= 2 ? 4 : NL <= 4 ? 2 : 1>(
+            G, t, parts,
             [&](int j, int i, float(&x)[2 * NL]) {
+                const int64_t o = G.x(j, i);
 #pragma unroll
                 for (int l = 0; l < NL; ++l) {
-                    x[l] = xbar[xidx(M, l, j, i)];
-                    x[NL + l] = direct ? direct[xidx(M, l, j, i)] : 0.f;
+                    x[l] = xbar[o + l * G.lx];
+                    x[NL + l] = direct ? direct[o + l * G.lx] : 0.f;
                 }
             },
             [&](int j, int i, float(&x)[2 * NL]) {
                 // q of the ring (under the BC) and of land cells is not read by the forward
-                const bool zero = (apply_bc && on_ring(j, i, M.Ny, M.Nx)) || is_land(M.mask, M.Ny, M.Nx, j, i);
+                const bool zero = (apply_bc && G.ring(j, i)) || G.land(j, i);
+                const int64_t c = G.c(j, i);
 #pragma unroll
                 for (int l = 0; l < NL; ++l) {
-                    float v = x[NL + l];
-#pragma unroll
-                    for (int m = 0; m < NL; ++m) v = fmaf(M.Cl2m[m * kMaxLayers + l], x[m], v);
-                    qbar[cidx(M, l, j, i)] = zero ? 0.f : v;
+                    const float v = C.row(l, x, x[NL + l]);
+                    qbar[c + l * G.lc] = zero ? 0.f : v;
                 }
             });
     });
@@ -301,15 +301,15 @@ cudaError_t launch_vjp_stencil(const VjpArgs& v, cudaStream_t s) {
 }
 
 cudaError_t launch_vjp_operand(const VjpArgs& v, const float* psi_bar, cudaStream_t s) {
-    const int parts = cell_parts(v.tile_x, v.ntiles);
-    return launch_k(k_vjp_operand, v.ntiles * parts, NT, 0, s, v.pdl, v.members, v.tiles, v.tile_x, v.tile_y, parts, v.rhs,
-                    psi_bar, v.xa, v.xa_fmt, v.xq, v.xplane);
+    const int parts = cell_parts(v.n_cells);
+    return launch_k(k_vjp_operand, v.n_cells * parts, NT, 0, s, v.pdl, v.members, v.cells, parts, v.rhs, psi_bar, v.xa,
+                    v.xa_fmt, v.xq, v.xplane);
 }
 
 cudaError_t launch_vjp_finish(const VjpArgs& v, const float* xbar, float* qbar, float* pbar, cudaStream_t s) {
-    const int parts = cell_parts(v.tile_x, v.ntiles);
-    cudaError_t e = launch_k(k_vjp_finish, v.ntiles * parts, NT, 0, s, v.pdl, v.members, v.tiles, v.tile_x, v.tile_y,
-                             parts, v.direct, xbar, v.apply_bc, qbar);
+    const int parts = cell_parts(v.n_cells);
+    cudaError_t e = launch_k(k_vjp_finish, v.n_cells * parts, NT, 0, s, v.pdl, v.members, v.cells, parts, v.direct, xbar,
+                             v.apply_bc, qbar);
     if (!e && pbar) {
         const int n = v.n_members * QG_NPARAMS;
         k_vjp_params<<<(n + 127) / 128, 128, 0, s>>>(v.pacc, n, pbar);

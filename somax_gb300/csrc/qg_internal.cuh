@@ -117,7 +117,7 @@ struct Tableau {
 
 struct PrepArgs {
     const MemberDev* members;
-    const StencilTile* tiles;
+    const StencilTile* tiles;  // 64 x 16
     const float* q;        // caller packing
     float* copy;           // internal x-row plane to receive q (may be null)
     int zero_ring_copy;    // zero the ring in the copy
@@ -126,15 +126,13 @@ struct PrepArgs {
     int xa_fmt;
     float* xq;             // FP32 Cl2m q for the refinement residual (may be null)
     int64_t xplane;
-    int tile_x, tile_y;    // cells per tile of the tile list
 };
 
 // Butcher-form stage combine: out = y0 + dt * sum_s coef[s] * k[s] and its modal operand.
 constexpr int kMaxStages = 8;
 struct RkCombineArgs {
     const MemberDev* members;
-    const StencilTile* tiles;
-    int tile_x, tile_y;
+    const StencilTile* tiles;  // 64 x 16
     const float* y0;       // x-row state plane
     const float* k;        // stage derivatives, caller packing, plane s at s * kplane
     int64_t kplane;
@@ -231,10 +229,10 @@ cudaError_t launch_lsweep_group(const StencilArgs& a, const SweepItem* items, in
 // launchers (return cudaError_t of the launch)
 cudaError_t launch_prep(const PrepArgs& a, int ntiles, cudaStream_t s, bool pdl);
 cudaError_t launch_write(float* dst, const float* values, int64_t n, cudaStream_t s);
-cudaError_t launch_unpack(const MemberDev* members, const StencilTile* tiles, int ntiles, int large,
-                          const float* src, float* q, cudaStream_t s, bool pdl);
-cudaError_t launch_mode_to_layer(const MemberDev* members, const StencilTile* tiles, int ntiles, int large,
-                                 const float* psi_hat, float* psi, cudaStream_t s, bool pdl);
+cudaError_t launch_unpack(const MemberDev* members, const StencilTile* tiles, int ntiles, const float* src, float* q,
+                          cudaStream_t s, bool pdl);
+cudaError_t launch_mode_to_layer(const MemberDev* members, const StencilTile* tiles, int ntiles, const float* psi_hat,
+                                 float* psi, cudaStream_t s, bool pdl);
 cudaError_t launch_diag_acc(const MemberDev* members, const StencilTile* tiles, int ntiles, int large,
                             const float* q, const float* psi_hat, double* acc, cudaStream_t s);
 // min / mean / max of the finite entries and the non-finite count of n floats into out[0..3]
@@ -254,15 +252,16 @@ cudaError_t launch_project_g_vjp(const MemberDev* members, const StencilTile* ti
                                  const float* hgb, const float* ugb, const float* vgb, float* psib, cudaStream_t s);
 cudaError_t launch_project_q_vjp(const MemberDev* members, const StencilTile* tiles, int ntiles, int large,
                                  const float* qb, float* hb, float* ub, float* vb, cudaStream_t s);
-cudaError_t launch_residual(const MemberDev* members, const StencilTile* tiles, int ntiles, int large,
-                            const float* qm, const float* psi_hat, void* out, int out_fmt,
-                            int64_t xplane, cudaStream_t s, bool pdl);
+cudaError_t launch_residual(const MemberDev* members, const StencilTile* tiles, int ntiles, const float* qm,
+                            const float* psi_hat, void* out, int out_fmt, int64_t xplane, cudaStream_t s, bool pdl);
 
 // Adjoint (qg_adjoint.cu): the RHS / inversion VJP around one adjoint DST solve.
 struct VjpArgs {
     const MemberDev* members;
     const StencilTile* tiles;
     int ntiles, tile_x, tile_y, max_nl, n_members;
+    const StencilTile* cells;  // 64 x 16 tiles of the kernels without a halo
+    int n_cells;
     const float* q;       // caller packing
     int apply_bc;         // the forward zeroed the ring of q on read
     const float* psi;     // layer psi of the forward, caller packing
@@ -500,8 +499,8 @@ int round_up(int v, int m);
 
 // stencil tile shapes (cells): small grids use 32 x 8, large ones 64 x 16
 constexpr int kTileSX = 32, kTileSY = 8, kTileLX = 64, kTileLY = 16;
-// CTAs per tile of the kernels that walk cells without a halo: the four passes of a large tile go to
-// four CTAs until a plan's tiles give every SM eight of them.
-constexpr int cell_parts(int tile_x, int ntiles) { return tile_x == kTileLX && ntiles < 8 * 152 ? 4 : 1; }
+// CTAs per 64 x 16 tile of the kernels that walk cells without a halo: its four passes go to four CTAs
+// until a plan's tiles give every SM eight of them.
+constexpr int cell_parts(int ntiles) { return ntiles < 8 * 152 ? 4 : 1; }
 
 }  // namespace qg

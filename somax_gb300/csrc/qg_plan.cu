@@ -484,7 +484,7 @@ cudaError_t run_dst_solve(qg_plan* p, cudaStream_t s) {
     if ((e = run_gemm(p, gemm_args(p, G4_INV_Y, p->YB, p->XC, f, FMT_F32, 0), s))) return e;
     for (int r = 0; r < p->opts.refine_sweeps; ++r) {
         e = timed(p, QG_K_OTHER, s, [&] {
-            return launch_residual(p->md, p->st_tiles, p->n_st, p->st_large, p->XQ, p->XC, p->XA, f, p->xplane, s,
+            return launch_residual(p->md, p->st_tiles_v[1], p->n_st_v[1], p->XQ, p->XC, p->XA, f, p->xplane, s,
                                    use_pdl(p));
         });
         if (e) return e;
@@ -503,6 +503,8 @@ VjpArgs vjp_args(qg_plan* p) {
     v.ntiles = p->n_st;
     v.tile_x = p->st_large ? kTileLX : kTileSX;
     v.tile_y = p->st_large ? kTileLY : kTileSY;
+    v.cells = p->st_tiles_v[1];
+    v.n_cells = p->n_st_v[1];
     v.max_nl = p->max_nl;
     v.n_members = p->n_members;
     v.pacc = p->vjp_acc;
@@ -545,7 +547,7 @@ cudaError_t run_prep(qg_plan* p, const float* q, float* copy, int zero_ring_copy
                      cudaStream_t s) {
     PrepArgs a{};
     a.members = p->md;
-    a.tiles = p->st_tiles;
+    a.tiles = p->st_tiles_v[1];
     a.q = q;
     a.copy = copy;
     a.zero_ring_copy = zero_ring_copy;
@@ -554,9 +556,7 @@ cudaError_t run_prep(qg_plan* p, const float* q, float* copy, int zero_ring_copy
     a.xa_fmt = p->op_fmt;
     a.xq = p->XQ;
     a.xplane = p->xplane;
-    a.tile_x = p->st_large ? kTileLX : kTileSX;
-    a.tile_y = p->st_large ? kTileLY : kTileSY;
-    return timed(p, QG_K_PREP, s, [&] { return launch_prep(a, p->n_st, s, use_pdl(p)); });
+    return timed(p, QG_K_PREP, s, [&] { return launch_prep(a, p->n_st_v[1], s, use_pdl(p)); });
 }
 
 StencilArgs stencil_args(qg_plan* p, const float* params) {
@@ -670,9 +670,7 @@ cudaError_t run_one_step_butcher(qg_plan* p, const float* params, float dt, cons
         if (e) break;
         RkCombineArgs c{};
         c.members = p->md;
-        c.tiles = p->st_tiles;
-        c.tile_x = p->st_large ? kTileLX : kTileSX;
-        c.tile_y = p->st_large ? kTileLY : kTileSY;
+        c.tiles = p->st_tiles_v[1];
         c.y0 = p->S0;
         c.k = p->K;
         c.kplane = p->state_size;
@@ -685,7 +683,7 @@ cudaError_t run_one_step_butcher(qg_plan* p, const float* params, float dt, cons
         c.xa_fmt = p->op_fmt;
         c.xq = p->XQ;
         c.xplane = p->xplane;
-        e = timed(p, QG_K_OTHER, s, [&] { return launch_rk_combine(c, p->n_st, s, use_pdl(p)); });
+        e = timed(p, QG_K_OTHER, s, [&] { return launch_rk_combine(c, p->n_st_v[1], s, use_pdl(p)); });
     }
     return e;
 }
@@ -1447,7 +1445,7 @@ int qg_invert(qg_plan* p, const float* q, float* psi, void* stream) {
     if (!e) e = run_inversion(p, s);
     if (!e)
         e = timed(p, QG_K_OTHER, s, [&] {
-            return launch_mode_to_layer(p->md, p->st_tiles, p->n_st, p->st_large, p->XC, psi, s, use_pdl(p));
+            return launch_mode_to_layer(p->md, p->st_tiles_v[1], p->n_st_v[1], p->XC, psi, s, use_pdl(p));
         });
     return cuda_err(e);
 }
@@ -1618,7 +1616,7 @@ int qg_step(qg_plan* p, float* q, const float* params, double dt, int n_steps, i
     }
     if (!e)
         e = timed(p, QG_K_OTHER, s, [&] {
-            return launch_unpack(p->md, p->st_tiles, p->n_st, p->st_large, p->S0, q, s, use_pdl(p));
+            return launch_unpack(p->md, p->st_tiles_v[1], p->n_st_v[1], p->S0, q, s, use_pdl(p));
         });
     return cuda_err(e);
 }
@@ -1637,7 +1635,7 @@ cudaError_t rhs_vjp_core(qg_plan* p, const float* q, const float* params, const 
         if (!e) e = run_inversion(p, s);
         if (!e)
             e = timed(p, QG_K_OTHER, s, [&] {
-                return launch_mode_to_layer(p->md, p->st_tiles, p->n_st, p->st_large, p->XC, p->YA, s, use_pdl(p));
+                return launch_mode_to_layer(p->md, p->st_tiles_v[1], p->n_st_v[1], p->XC, p->YA, s, use_pdl(p));
             });
         psi = p->YA;
     }
@@ -1704,7 +1702,7 @@ cudaError_t step_vjp_body(qg_plan* p, const float* y0, const float* params, doub
         // psi_hat of B(Y_{st-1}) is still in XC: keep its layer psi for the reverse sweep
         if (!e)
             e = timed(p, QG_K_OTHER, s, [&] {
-                return launch_mode_to_layer(p->md, p->st_tiles, p->n_st, p->st_large, p->XC, Psi[st - 1], s,
+                return launch_mode_to_layer(p->md, p->st_tiles_v[1], p->n_st_v[1], p->XC, Psi[st - 1], s,
                                             use_pdl(p));
             });
         float c[kMaxButcher];
@@ -1804,7 +1802,7 @@ int qg_diagnose_fields(qg_plan* p, const float* q, float* psi, float* u, float* 
     if (!e) e = run_inversion(p, s);
     if (!e)
         e = timed(p, QG_K_OTHER, s, [&] {
-            return launch_mode_to_layer(p->md, p->st_tiles, p->n_st, p->st_large, p->XC, psi, s, false);
+            return launch_mode_to_layer(p->md, p->st_tiles_v[1], p->n_st_v[1], p->XC, psi, s, false);
         });
     if (!e)
         e = timed(p, QG_K_OTHER, s, [&] {

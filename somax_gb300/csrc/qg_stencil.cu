@@ -22,63 +22,67 @@ using namespace st;
 // Pack: copy q (caller packing) into an internal plane (optionally zeroing its ring) and
 // write the layer->mode operand Cl2m q (BC applied when bc_operand) for the DST GEMMs.
 // ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(NTHREADS) k_prep(PrepArgs a, int parts) {
+__global__ void __launch_bounds__(NTHREADS, 4) k_prep(PrepArgs a, int parts) {
     __shared__ MemberDev M;
     const StencilTile t = a.tiles[blockIdx.x / (unsigned)parts];
     load_member(&M, a.members + t.member);
     __syncthreads();
     pdl_wait();
     pdl_launch_dependents();
+    const CellGeom G(M);
     with_layers(M.nl, [&](auto n) {
         constexpr int NL = decltype(n)::value;
+        const Mix<NL> C(M.Cl2m);
         walk_cells<NL, NL <= 4 ? 4 : 2>(
-            M, t, a.tile_x, a.tile_y, parts,
+            G, t, parts,
             [&](int j, int i, float(&x)[NL]) {
+                const int64_t o = G.c(j, i);
 #pragma unroll
-                for (int l = 0; l < NL; ++l) x[l] = a.q[caller_idx(M, l, j, i)];
+                for (int l = 0; l < NL; ++l) x[l] = a.q[o + l * G.lc];
             },
             [&](int j, int i, float(&x)[NL]) {
-                const bool ring = on_ring(j, i, M.Ny, M.Nx);
-                const bool land = is_land(M, j, i);  // q reads as zero on land
+                const bool ring = G.ring(j, i), land = G.land(j, i);  // q reads as zero on land
+                const int64_t o = G.x(j, i);
 #pragma unroll
                 for (int l = 0; l < NL; ++l) {
-                    if (a.copy) a.copy[xrow_idx(M, l, j, i)] = (a.zero_ring_copy && (ring || land)) ? 0.f : x[l];
+                    if (a.copy) a.copy[o + l * G.lx] = (a.zero_ring_copy && (ring || land)) ? 0.f : x[l];
                     x[l] = ((a.bc_operand && ring) || land) ? 0.f : x[l];
                 }
                 if (!a.xa) return;
 #pragma unroll
                 for (int m = 0; m < NL; ++m) {
-                    float s = 0.f;
-#pragma unroll
-                    for (int l = 0; l < NL; ++l) s = fmaf(M.Cl2m[m * kMaxLayers + l], x[l], s);
-                    store_plane(a.xa, a.xa_fmt, a.xplane, xrow_idx(M, m, j, i), s);
-                    if (a.xq) a.xq[xrow_idx(M, m, j, i)] = s;
+                    const float s = C.row(m, x);
+                    store_plane(a.xa, a.xa_fmt, a.xplane, o + m * G.lx, s);
+                    if (a.xq) a.xq[o + m * G.lx] = s;
                 }
             });
     });
 }
 
 // Unpack: internal plane -> caller packing (every cell, ring included).
-__global__ void __launch_bounds__(NTHREADS) k_unpack(const MemberDev* __restrict__ members,
-                                                     const StencilTile* __restrict__ tiles, int TX, int TY, int parts,
-                                                     const float* src, float* q) {
+__global__ void __launch_bounds__(NTHREADS, 4) k_unpack(const MemberDev* __restrict__ members,
+                                                     const StencilTile* __restrict__ tiles, int parts, const float* src,
+                                                     float* q) {
     __shared__ MemberDev M;
     const StencilTile t = tiles[blockIdx.x / (unsigned)parts];
     load_member(&M, members + t.member);
     __syncthreads();
     pdl_wait();
     pdl_launch_dependents();
+    const CellGeom G(M);
     with_layers(M.nl, [&](auto n) {
         constexpr int NL = decltype(n)::value;
         walk_cells<NL, NL <= 4 ? 4 : 2>(
-            M, t, TX, TY, parts,
+            G, t, parts,
             [&](int j, int i, float(&x)[NL]) {
+                const int64_t o = G.x(j, i);
 #pragma unroll
-                for (int l = 0; l < NL; ++l) x[l] = src[xrow_idx(M, l, j, i)];
+                for (int l = 0; l < NL; ++l) x[l] = src[o + l * G.lx];
             },
             [&](int j, int i, float(&x)[NL]) {
+                const int64_t o = G.c(j, i);
 #pragma unroll
-                for (int l = 0; l < NL; ++l) q[caller_idx(M, l, j, i)] = x[l];
+                for (int l = 0; l < NL; ++l) q[o + l * G.lc] = x[l];
             });
     });
 }
@@ -90,46 +94,46 @@ __global__ void __launch_bounds__(NTHREADS) k_unpack(const MemberDev* __restrict
 // solve.  The ring is combined like every other cell; stage inputs are read with the BC, and
 // the final combination's ring is y0 + dt * wind as in the fused Shu-Osher stencil.
 // ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(NTHREADS) k_rk_combine(RkCombineArgs a, int parts) {
+__global__ void __launch_bounds__(NTHREADS, 4) k_rk_combine(RkCombineArgs a, int parts) {
     __shared__ MemberDev M;
     const StencilTile t = a.tiles[blockIdx.x / (unsigned)parts];
     load_member(&M, a.members + t.member);
     __syncthreads();
     pdl_wait();
     pdl_launch_dependents();
+    const CellGeom G(M);
     with_layers(M.nl, [&](auto n) {
         constexpr int NL = decltype(n)::value;
+        const Mix<NL> C(M.Cl2m);
         walk_cells<NL, NL <= 2 ? 4 : NL <= 4 ? 2 : 1>(
-            M, t, a.tile_x, a.tile_y, parts,
+            G, t, parts,
             [&](int j, int i, float(&v)[NL]) {
-                const int64_t ci = caller_idx(M, 0, j, i), cl = (int64_t)M.Ny * M.Nx;
+                const int64_t ci = G.c(j, i), xi = G.x(j, i);
                 float acc[NL];
 #pragma unroll
                 for (int l = 0; l < NL; ++l) {
                     acc[l] = 0.f;
-                    v[l] = a.y0[xrow_idx(M, l, j, i)];
+                    v[l] = a.y0[xi + l * G.lx];
                 }
 #pragma unroll
                 for (int s = 0; s < kMaxButcher; ++s)
                     if (s < a.n_k && a.coef[s] != 0.f)
 #pragma unroll
                         for (int l = 0; l < NL; ++l)
-                            acc[l] = fmaf(a.coef[s], a.k[(int64_t)s * a.kplane + ci + l * cl], acc[l]);
+                            acc[l] = fmaf(a.coef[s], a.k[(int64_t)s * a.kplane + ci + l * G.lc], acc[l]);
 #pragma unroll
                 for (int l = 0; l < NL; ++l) v[l] += a.dt * acc[l];
             },
             [&](int j, int i, float(&v)[NL]) {
-                const bool zero = on_ring(j, i, M.Ny, M.Nx) || is_land(M, j, i);
+                const bool zero = G.ring(j, i) || G.land(j, i);
+                const int64_t xi = G.x(j, i);
 #pragma unroll
-                for (int l = 0; l < NL; ++l) a.out[xrow_idx(M, l, j, i)] = v[l];
+                for (int l = 0; l < NL; ++l) a.out[xi + l * G.lx] = v[l];
 #pragma unroll
                 for (int m = 0; m < NL; ++m) {
-                    float sum = 0.f;
-                    if (!zero)
-#pragma unroll
-                        for (int l = 0; l < NL; ++l) sum = fmaf(M.Cl2m[m * kMaxLayers + l], v[l], sum);
-                    store_plane(a.xa, a.xa_fmt, a.xplane, xrow_idx(M, m, j, i), sum);
-                    if (a.xq) a.xq[xrow_idx(M, m, j, i)] = sum;
+                    const float sum = zero ? 0.f : C.row(m, v);
+                    store_plane(a.xa, a.xa_fmt, a.xplane, xi + m * G.lx, sum);
+                    if (a.xq) a.xq[xi + m * G.lx] = sum;
                 }
             });
     });
@@ -138,32 +142,32 @@ __global__ void __launch_bounds__(NTHREADS) k_rk_combine(RkCombineArgs a, int pa
 // ---------------------------------------------------------------------------------------
 // Mode -> layer epilogue for qg_invert: psi = Cm2l psi_hat, ring zeroed (baroclinic).
 // ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(NTHREADS) k_mode_to_layer(const MemberDev* __restrict__ members,
-                                                            const StencilTile* __restrict__ tiles, int TX, int TY,
-                                                            int parts, const float* psi_hat, float* psi) {
+__global__ void __launch_bounds__(NTHREADS, 4) k_mode_to_layer(const MemberDev* __restrict__ members,
+                                                            const StencilTile* __restrict__ tiles, int parts,
+                                                            const float* psi_hat, float* psi) {
     __shared__ MemberDev M;
     const StencilTile t = tiles[blockIdx.x / (unsigned)parts];
     load_member(&M, members + t.member);
     __syncthreads();
     pdl_wait();
     pdl_launch_dependents();
+    const CellGeom G(M);
     with_layers(M.nl, [&](auto n) {
         constexpr int NL = decltype(n)::value;
-        walk_cells<NL, NL <= 4 ? 4 : 2>(
-            M, t, TX, TY, parts,
+        const Mix<NL> C(M.Cm2l);
+        const bool keep_ring = M.barotropic;
+        walk_cells<NL, NL <= 4 ? 4 : 1>(
+            G, t, parts,
             [&](int j, int i, float(&x)[NL]) {
+                const int64_t o = G.x(j, i);
 #pragma unroll
-                for (int m = 0; m < NL; ++m) x[m] = psi_hat[xrow_idx(M, m, j, i)];
+                for (int m = 0; m < NL; ++m) x[m] = psi_hat[o + m * G.lx];
             },
             [&](int j, int i, float(&x)[NL]) {
-                const bool zero = (!M.barotropic && on_ring(j, i, M.Ny, M.Nx)) || is_land(M, j, i);
+                const bool zero = (!keep_ring && G.ring(j, i)) || G.land(j, i);
+                const int64_t o = G.c(j, i);
 #pragma unroll
-                for (int l = 0; l < NL; ++l) {
-                    float p = 0.f;
-#pragma unroll
-                    for (int m = 0; m < NL; ++m) p = fmaf(M.Cm2l[l * kMaxLayers + m], x[m], p);
-                    psi[caller_idx(M, l, j, i)] = zero ? 0.f : p;
-                }
+                for (int l = 0; l < NL; ++l) psi[o + l * G.lc] = zero ? 0.f : C.row(l, x);
             });
     });
 }
@@ -315,33 +319,39 @@ __global__ void __launch_bounds__(NTHREADS) k_project_q_vjp(const MemberDev* __r
 // where lap_full is the full-array 5-point operator with zeros outside the array (the
 // operator the DST-I solve inverts).  qm is the FP32 modal right-hand side.
 // ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(NTHREADS) k_residual(const MemberDev* __restrict__ members,
-                                                       const StencilTile* __restrict__ tiles, int TX, int TY, int parts,
-                                                       const float* qm, const float* psi_hat, void* out, int out_fmt,
-                                                       int64_t xplane) {
+__global__ void __launch_bounds__(NTHREADS, 4) k_residual(const MemberDev* __restrict__ members,
+                                                       const StencilTile* __restrict__ tiles, int parts, const float* qm,
+                                                       const float* psi_hat, void* out, int out_fmt, int64_t xplane) {
     __shared__ MemberDev M;
     const StencilTile t = tiles[blockIdx.x / (unsigned)parts];
     load_member(&M, members + t.member);
     __syncthreads();
     pdl_wait();
     pdl_launch_dependents();
+    const CellGeom G(M);
     with_layers(M.nl, [&](auto n) {
         constexpr int NL = decltype(n)::value;
+        const float idx2 = M.inv_dx2, idy2 = M.inv_dy2;
+        float lam[NL];
+#pragma unroll
+        for (int m = 0; m < NL; ++m) lam[m] = M.lam[m];
         walk_cells<NL, NL <= 2 ? 2 : 1>(
-            M, t, TX, TY, parts,
+            G, t, parts,
             [&](int j, int i, float(&r)[NL]) {
+                const int64_t o = G.x(j, i);
 #pragma unroll
                 for (int m = 0; m < NL; ++m) {
-                    const float* p = psi_hat + xrow_idx(M, m, j, i);
-                    const float c0 = p[0], e = i + 1 < M.Nx ? p[1] : 0.f, w = i > 0 ? p[-1] : 0.f;
-                    const float no = j + 1 < M.Ny ? p[M.Px] : 0.f, so = j > 0 ? p[-M.Px] : 0.f;
-                    const float lap = (e - 2.f * c0 + w) * M.inv_dx2 + (no - 2.f * c0 + so) * M.inv_dy2;
-                    r[m] = qm[xrow_idx(M, m, j, i)] - (lap - M.lam[m] * c0);
+                    const float* p = psi_hat + o + m * G.lx;
+                    const float c0 = p[0], e = i + 1 < G.Nx ? p[1] : 0.f, w = i > 0 ? p[-1] : 0.f;
+                    const float no = j + 1 < G.Ny ? p[G.Px] : 0.f, so = j > 0 ? p[-G.Px] : 0.f;
+                    const float lap = (e - 2.f * c0 + w) * idx2 + (no - 2.f * c0 + so) * idy2;
+                    r[m] = qm[o + m * G.lx] - (lap - lam[m] * c0);
                 }
             },
             [&](int j, int i, float(&r)[NL]) {
+                const int64_t o = G.x(j, i);
 #pragma unroll
-                for (int m = 0; m < NL; ++m) store_plane(out, out_fmt, xplane, xrow_idx(M, m, j, i), r[m]);
+                for (int m = 0; m < NL; ++m) store_plane(out, out_fmt, xplane, o + m * G.lx, r[m]);
             });
     });
 }
@@ -583,12 +593,12 @@ cudaError_t stencil_encode_maps(const MemberDev& M, const float* const planes[4]
 }
 
 cudaError_t launch_prep(const PrepArgs& a, int ntiles, cudaStream_t s, bool pdl) {
-    const int parts = cell_parts(a.tile_x, ntiles);
+    const int parts = cell_parts(ntiles);
     return launch_k(k_prep, ntiles * parts, NTHREADS, 0, s, pdl, a, parts);
 }
 
 cudaError_t launch_rk_combine(const RkCombineArgs& a, int ntiles, cudaStream_t s, bool pdl) {
-    const int parts = cell_parts(a.tile_x, ntiles);
+    const int parts = cell_parts(ntiles);
     return launch_k(k_rk_combine, ntiles * parts, NTHREADS, 0, s, pdl, a, parts);
 }
 
@@ -620,16 +630,16 @@ cudaError_t launch_write(float* dst, const float* values, int64_t n, cudaStream_
     return e;
 }
 
-cudaError_t launch_unpack(const MemberDev* members, const StencilTile* tiles, int ntiles, int large,
-                          const float* src, float* q, cudaStream_t s, bool pdl) {
-    const int tx = large ? TileL::TX : TileS::TX, ty = large ? TileL::TY : TileS::TY, parts = cell_parts(tx, ntiles);
-    return launch_k(k_unpack, ntiles * parts, NTHREADS, 0, s, pdl, members, tiles, tx, ty, parts, src, q);
+cudaError_t launch_unpack(const MemberDev* members, const StencilTile* tiles, int ntiles, const float* src, float* q,
+                          cudaStream_t s, bool pdl) {
+    const int parts = cell_parts(ntiles);
+    return launch_k(k_unpack, ntiles * parts, NTHREADS, 0, s, pdl, members, tiles, parts, src, q);
 }
 
-cudaError_t launch_mode_to_layer(const MemberDev* members, const StencilTile* tiles, int ntiles, int large,
-                                 const float* psi_hat, float* psi, cudaStream_t s, bool pdl) {
-    const int tx = large ? TileL::TX : TileS::TX, ty = large ? TileL::TY : TileS::TY, parts = cell_parts(tx, ntiles);
-    return launch_k(k_mode_to_layer, ntiles * parts, NTHREADS, 0, s, pdl, members, tiles, tx, ty, parts, psi_hat, psi);
+cudaError_t launch_mode_to_layer(const MemberDev* members, const StencilTile* tiles, int ntiles, const float* psi_hat,
+                                 float* psi, cudaStream_t s, bool pdl) {
+    const int parts = cell_parts(ntiles);
+    return launch_k(k_mode_to_layer, ntiles * parts, NTHREADS, 0, s, pdl, members, tiles, parts, psi_hat, psi);
 }
 
 cudaError_t launch_project_q(const MemberDev* members, const StencilTile* tiles, int ntiles, int large,
@@ -656,12 +666,11 @@ cudaError_t launch_project_q_vjp(const MemberDev* members, const StencilTile* ti
                     large ? TileL::TY : TileS::TY, qb, hb, ub, vb);
 }
 
-cudaError_t launch_residual(const MemberDev* members, const StencilTile* tiles, int ntiles, int large,
-                            const float* qm, const float* psi_hat, void* out, int out_fmt,
-                            int64_t xplane, cudaStream_t s, bool pdl) {
-    const int tx = large ? TileL::TX : TileS::TX, ty = large ? TileL::TY : TileS::TY, parts = cell_parts(tx, ntiles);
-    return launch_k(k_residual, ntiles * parts, NTHREADS, 0, s, pdl, members, tiles, tx, ty, parts, qm, psi_hat, out,
-                    out_fmt, xplane);
+cudaError_t launch_residual(const MemberDev* members, const StencilTile* tiles, int ntiles, const float* qm,
+                            const float* psi_hat, void* out, int out_fmt, int64_t xplane, cudaStream_t s, bool pdl) {
+    const int parts = cell_parts(ntiles);
+    return launch_k(k_residual, ntiles * parts, NTHREADS, 0, s, pdl, members, tiles, parts, qm, psi_hat, out, out_fmt,
+                    xplane);
 }
 
 cudaError_t launch_diag_acc(const MemberDev* members, const StencilTile* tiles, int ntiles, int large,

@@ -97,22 +97,63 @@ __device__ __forceinline__ void with_layers(int nl, F&& f) {
     }
 }
 
+// What the kernels without a halo take from a member, in registers (their stores may alias the shared
+// copy, which the compiler would read again after each): index bases and strides in the caller's
+// packing and the x-row planes, and the mixing matrix of up to four layers.
+struct CellGeom {
+    int64_t oc, ox, lc, lx;
+    int Ny, Nx, Px;
+    const uint8_t* mask;
+    __device__ __forceinline__ explicit CellGeom(const MemberDev& M)
+        : oc(M.off_state), ox(M.off_x), lc((int64_t)M.Ny * M.Nx), lx((int64_t)M.Ny * M.Px), Ny(M.Ny), Nx(M.Nx), Px(M.Px),
+          mask(M.mask) {}
+    __device__ __forceinline__ int64_t c(int j, int i) const { return oc + (int64_t)j * Nx + i; }  // + l * lc
+    __device__ __forceinline__ int64_t x(int j, int i) const { return ox + (int64_t)j * Px + i; }  // + l * lx
+    __device__ __forceinline__ bool ring(int j, int i) const { return on_ring(j, i, Ny, Nx); }
+    __device__ __forceinline__ bool land(int j, int i) const { return is_land(mask, Ny, Nx, j, i); }
+};
+template <int NL, bool T = false>  // T: the transposed matrix
+struct Mix {
+    static constexpr bool kHeld = NL <= 4;  // larger ones stay in shared memory: 64 registers a thread
+    float held[kHeld ? NL : 1][kHeld ? NL : 1];
+    const float* m;
+    __device__ __forceinline__ explicit Mix(const float* mat) : m(mat) {
+        if constexpr (kHeld)
+#pragma unroll
+            for (int r = 0; r < NL; ++r)
+#pragma unroll
+                for (int c = 0; c < NL; ++c) held[r][c] = m[T ? c * kMaxLayers + r : r * kMaxLayers + c];
+    }
+    __device__ __forceinline__ float at(int r, int c) const {
+        if constexpr (kHeld)
+            return held[r][c];
+        else
+            return m[T ? c * kMaxLayers + r : r * kMaxLayers + c];
+    }
+    template <int N>
+    __device__ __forceinline__ float row(int r, const float (&x)[N], float s = 0.f) const {
+#pragma unroll
+        for (int c = 0; c < NL; ++c) s = fmaf(at(r, c), x[c], s);
+        return s;
+    }
+};
+
 // The cells of a tile for a kernel without a halo: NL values x of a cell from load(j, i, x), then
 // use(j, i, x).  Bound: HBM on large plans, latency on small ones.  Loops over a layer count known
 // at run time kept one or two loads of a thread in flight; here every load of UNR cells, all layers,
-// is issued before the first store.  `parts` CTAs share a tile (cell_parts).
+// is issued before the first store.  Tiles are 64 x 16 whatever shape the stencil runs (a CTA of
+// 32 x 8 cells spends as long on its member's constants); `parts` CTAs share one (cell_parts).
 template <int NL, int UNR, class Load, class Use>
-__device__ __forceinline__ void walk_cells(const MemberDev& M, const StencilTile& t, int TX, int TY, int parts,
-                                           Load&& load, Use&& use) {
-    const int sh = TX == kTileLX ? 6 : 5, step = NTHREADS * parts;
-    static_assert(kTileLX == 64 && kTileSX == 32, "tile columns by shift");
+__device__ __forceinline__ void walk_cells(const CellGeom& G, const StencilTile& t, int parts, Load&& load, Use&& use) {
+    constexpr int TX = kTileLX, TY = kTileLY;
+    const int step = NTHREADS * parts;
     for (int c0 = threadIdx.x + (int)(blockIdx.x % (unsigned)parts) * NTHREADS; c0 < TX * TY; c0 += UNR * step) {
         float x[UNR][NL];
         auto at = [&](int u, int& j, int& i) {
             const int c = c0 + u * step;
-            j = t.ty * TY + (c >> sh);
-            i = t.tx * TX + (c & (TX - 1));
-            return c < TX * TY && j < M.Ny && i < M.Nx;
+            j = t.ty * TY + c / TX;
+            i = t.tx * TX + c % TX;
+            return c < TX * TY && j < G.Ny && i < G.Nx;
         };
 #pragma unroll
         for (int u = 0; u < UNR; ++u) {
