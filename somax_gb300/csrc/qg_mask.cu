@@ -61,7 +61,9 @@ __global__ void __launch_bounds__(NT) k_capacitance(const MemberDev* members, co
         // accumulate: a repeated correction adds to the sources already at B
         const int b = M.bidx[r];
         const int64_t o = M.off_x + ((int64_t)m * M.Ny + b / Nx) * M.Px + (b % Nx);
-        if (xa_fmt == FMT_F32) {
+        if (!xa) {
+            // the refinement's residual forms the operand from xq
+        } else if (xa_fmt == FMT_F32) {
             float* p = static_cast<float*>(xa);
             p[o] = (float)((double)p[o] - s);
         } else {

@@ -473,27 +473,31 @@ cudaError_t run_cols(qg_plan* p, cudaStream_t s) {
     c.V = p->XA;
     return timed(p, QG_K_GEMM, s, [&] { return launch_cols(c, p->n_members, s, use_pdl(p)); });
 }
-// psi_hat (XC) from the modal operand already in XA (and XQ for refinement).
-cudaError_t run_dst_solve(qg_plan* p, cudaStream_t s) {
+// The four passes: psi_hat (XC) from the modal operand in XA, added to what XC holds if accumulate.
+cudaError_t run_passes(qg_plan* p, int accumulate, cudaStream_t s) {
     const int f = p->op_fmt;
     cudaError_t e;
     // the last pass writes FP32 psi_hat; intermediate planes use the operand format
     if ((e = run_gemm(p, gemm_args(p, G1_FWD_X, p->XA, p->YA, f, f, 0), s))) return e;
     if ((e = run_gemm(p, gemm_args(p, G2_FWD_Y, p->YA, p->XB, f, f, 0), s))) return e;
     if ((e = run_gemm(p, gemm_args(p, G3_INV_X, p->XB, p->YB, f, f, 0), s))) return e;
-    if ((e = run_gemm(p, gemm_args(p, G4_INV_Y, p->YB, p->XC, f, FMT_F32, 0), s))) return e;
-    for (int r = 0; r < p->opts.refine_sweeps; ++r) {
-        e = timed(p, QG_K_OTHER, s, [&] {
-            return launch_residual(p->md, p->st_tiles_v[1], p->n_st_v[1], p->XQ, p->XC, p->XA, f, p->xplane, s,
-                                   use_pdl(p));
-        });
-        if (e) return e;
-        if ((e = run_gemm(p, gemm_args(p, G1_FWD_X, p->XA, p->YA, f, f, 0), s))) return e;
-        if ((e = run_gemm(p, gemm_args(p, G2_FWD_Y, p->YA, p->XB, f, f, 0), s))) return e;
-        if ((e = run_gemm(p, gemm_args(p, G3_INV_X, p->XB, p->YB, f, f, 0), s))) return e;
-        if ((e = run_gemm(p, gemm_args(p, G4_INV_Y, p->YB, p->XC, f, FMT_F32, 1), s))) return e;
-    }
-    return cudaSuccess;
+    return run_gemm(p, gemm_args(p, G4_INV_Y, p->YB, p->XC, f, FMT_F32, accumulate), s);
+}
+
+// psi_hat += the solve of the residual of the right-hand side in XQ.
+cudaError_t run_refine(qg_plan* p, cudaStream_t s) {
+    const cudaError_t e = timed(p, QG_K_OTHER, s, [&] {
+        return launch_residual(p->md, p->st_tiles_v[1], p->n_st_v[1], p->XQ, p->XC, p->XA, p->op_fmt, p->xplane, s,
+                               use_pdl(p));
+    });
+    return e ? e : run_passes(p, 1, s);
+}
+
+// psi_hat (XC) from the modal operand already in XA (and XQ for refinement).
+cudaError_t run_dst_solve(qg_plan* p, cudaStream_t s) {
+    cudaError_t e = run_passes(p, 0, s);
+    for (int r = 0; r < p->opts.refine_sweeps && !e; ++r) e = run_refine(p, s);
+    return e;
 }
 
 VjpArgs vjp_args(qg_plan* p) {
@@ -516,28 +520,27 @@ VjpArgs vjp_args(qg_plan* p) {
     return v;
 }
 
-// psi_hat (XC) with the masked members' capacitance correction: solve, sigma at B into the
-// operand, solve again (the operand is otherwise unchanged: it is zero on land).  With
-// refinement the correction repeats once more, so that psi on B falls to the solve's
-// precision squared (the FP64 capacitance matrices are exact, the solves are not).
+// psi_hat (XC) with the masked members' capacitance correction.  Without refinement: solve, sigma at
+// B into the operand, solve again (the operand is otherwise unchanged: it is zero on land).  With it
+// the corrections are sweeps of the refinement: sigma goes into the FP32 right-hand side, and the
+// residual's solve is added to psi.  With a solve of relative error eps, sweep k leaves
+//   e_k+1 = delta r_k,  b_k+1 = -e_k + delta r_k   (|delta| = eps, r_k of the size of e_k and b_k)
+// of the solve's error e and of psi on B, so that three sweeps after the first solve bring both to
+// eps^2 (e_0 = eps, b_0 = 1), FP32's rounding for FP32 and split BF16.  Refining a solve from scratch
+// after each of two corrections took six solves and not four for that: 193 us a stage at 250 x 190 x 3,
+// now 152.  TF32, whose eps the corrections amplify to 0.1, spends the six: five sweeps leave 1e-6 to
+// 2e-5 of psi where six solves left 1e-5 to 6e-4.
 cudaError_t run_inversion(qg_plan* p, cudaStream_t s) {
-    cudaError_t e = run_dst_solve(p, s);
-    if (e || p->n_cap == 0) return e;
-    for (int c = 0; c < 1 + p->opts.refine_sweeps && !e; ++c) {
+    if (p->n_cap == 0) return run_dst_solve(p, s);
+    cudaError_t e = run_passes(p, 0, s);
+    const int sweeps = p->opts.refine_sweeps == 0 ? 1 : p->opts.dst_precision == QG_DST_TF32 ? 5 : 3;
+    for (int c = 0; c < sweeps && !e; ++c) {
+        const bool refine = p->opts.refine_sweeps > 0;
         e = timed(p, QG_K_OTHER, s, [&] {
-            return launch_capacitance(p->md, p->cap_items, p->n_cap, p->XC, p->XA, p->op_fmt, p->XQ, p->xplane,
-                                      p->cap_smem, s, use_pdl(p));
+            return launch_capacitance(p->md, p->cap_items, p->n_cap, p->XC, refine ? nullptr : p->XA, p->op_fmt, p->XQ,
+                                      p->xplane, p->cap_smem, s, use_pdl(p));
         });
-        // a refinement sweep leaves its residual in the operand: rebuild it from the FP32
-        // right-hand side (which holds the sources on B)
-        if (!e && p->opts.refine_sweeps > 0)
-            e = timed(p, QG_K_PREP, s, [&] {
-                VjpArgs v = vjp_args(p);
-                v.rhs = p->XQ;
-                v.xq = nullptr;
-                return launch_vjp_operand(v, nullptr, s);
-            });
-        if (!e) e = run_dst_solve(p, s);
+        if (!e) e = refine ? run_refine(p, s) : run_passes(p, 0, s);
     }
     return e;
 }

@@ -14,7 +14,7 @@ from test_gpu_masked import RTOL_MASK, cuda, field, pair, rel
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("precision,refine", [("fp32", 0), ("bf16x3", 1)])
+@pytest.mark.parametrize("precision,refine", [("fp32", 0), ("fp32", 1), ("bf16x3", 1), ("tf32", 1)])
 @pytest.mark.parametrize("n", [1, 7, 8, 9, 511, 512, 513, 700])
 def test_boundary_points(n, precision, refine):
     nx, ny, nl = 62, 50, 2
