@@ -258,17 +258,14 @@ cudaError_t launch_residual(const MemberDev* members, const StencilTile* tiles, 
 // Adjoint (qg_adjoint.cu): the RHS / inversion VJP around one adjoint DST solve.
 struct VjpArgs {
     const MemberDev* members;
-    const StencilTile* tiles;
-    int ntiles, tile_x, tile_y, max_nl, n_members;
-    const StencilTile* cells;  // 64 x 16 tiles of the kernels without a halo
-    int n_cells;
+    const StencilTile* cells;  // 64 x 16 tiles
+    int n_cells, max_nl, n_members;
     const float* q;       // caller packing
     int apply_bc;         // the forward zeroed the ring of q on read
     const float* psi;     // layer psi of the forward, caller packing
     const float* gbar;    // cotangent of dq, caller packing
     const float* params;  // n_members * QG_NPARAMS
     float* direct;        // x-row plane: cotangent of qb from the stencil terms (null: none)
-    float* rhs;           // FP32 x-row modal plane: Cm2l^T Z psi_bar (zeroed before the stencil)
     double* pacc;         // parameter cotangents (zeroed before the stencil)
     void* xa;             // GEMM operand of the adjoint solve
     int xa_fmt;
@@ -278,14 +275,15 @@ struct VjpArgs {
 };
 cudaError_t launch_vjp_stencil(const VjpArgs& v, cudaStream_t s);
 cudaError_t launch_vjp_operand(const VjpArgs& v, const float* psi_bar, cudaStream_t s);
-cudaError_t launch_vjp_finish(const VjpArgs& v, const float* xbar, float* qbar, float* pbar, cudaStream_t s);
+cudaError_t launch_vjp_finish(const VjpArgs& v, const float* xbar, float* qbar, cudaStream_t s);
+cudaError_t launch_vjp_scatter(const VjpArgs& v, const float* xbar, float* ybar, float* const* kbar, const float* c,
+                               int n_terms, cudaStream_t s);
 cudaError_t launch_vjp_params_only(const VjpArgs& v, float* pbar, cudaStream_t s);
-// out = base + sum_j c_j x_j; ybar += Yb, kbar_j += c_j Yb; out_j = c_j g (n floats each)
+// out = base + sum_j c_j x_j; out_j = c_j g and acc = 0 (n floats each, n_acc sums)
 cudaError_t launch_lincomb(float* out, const float* base, const float* const* x, const float* c, int n_terms,
-                           int64_t n, cudaStream_t s);
-cudaError_t launch_scatter_bar(float* ybar, const float* Yb, float* const* kbar, const float* c, int n_terms,
-                               int64_t n, cudaStream_t s);
-cudaError_t launch_fanout(const float* g, float* const* out, const float* c, int n_terms, int64_t n, cudaStream_t s);
+                           int64_t n, cudaStream_t s, bool pdl);
+cudaError_t launch_fanout(const float* g, float* const* out, const float* c, int n_terms, int64_t n, double* acc,
+                          int n_acc, cudaStream_t s, bool pdl);
 const Tableau* swm_tableau(int scheme);
 
 // host: cuTensorMapEncodeTiled through the driver entry point (no libcuda link needed)

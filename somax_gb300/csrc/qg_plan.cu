@@ -503,10 +503,6 @@ cudaError_t run_dst_solve(qg_plan* p, cudaStream_t s) {
 VjpArgs vjp_args(qg_plan* p) {
     VjpArgs v{};
     v.members = p->md;
-    v.tiles = p->st_tiles;
-    v.ntiles = p->n_st;
-    v.tile_x = p->st_large ? kTileLX : kTileSX;
-    v.tile_y = p->st_large ? kTileLY : kTileSY;
     v.cells = p->st_tiles_v[1];
     v.n_cells = p->n_st_v[1];
     v.max_nl = p->max_nl;
@@ -1625,11 +1621,12 @@ int qg_step(qg_plan* p, float* q, const float* params, double dt, int n_steps, i
 }
 
 namespace {
-// q_bar = (d dq / d q)^T dq_bar of the rhs at q; the parameter cotangents are added to the
-// plan's FP64 accumulators (zeroed by the caller).  psi: the layer psi of q (caller packing)
-// when the caller has it, else null (computed here).
-cudaError_t rhs_vjp_core(qg_plan* p, const float* q, const float* params, const float* dq_bar, float* q_bar,
-                         int bc, cudaStream_t s, const float* psi = nullptr) {
+// The adjoint solve of the rhs at q for the cotangent dq_bar (its output in XC, the direct cotangent
+// of q in S2; *v: the arguments that launch_vjp_finish or _scatter needs); the parameter cotangents are
+// added to the plan's FP64 accumulators (zeroed by the caller).  psi: the layer psi of q (caller
+// packing) when the caller has it, else null (computed here).
+cudaError_t rhs_vjp_core(qg_plan* p, const float* q, const float* params, const float* dq_bar, int bc, cudaStream_t s,
+                         const float* psi, VjpArgs* v) {
     cudaError_t e = cudaSuccess;
     if (!psi) {
         // forward psi (layer, caller packing) into the YA plane, which holds at least one field
@@ -1642,21 +1639,16 @@ cudaError_t rhs_vjp_core(qg_plan* p, const float* q, const float* params, const 
             });
         psi = p->YA;
     }
-    // stencil transposes: direct cotangent into S2, the adjoint solve's modal rhs into XB
-    VjpArgs v = vjp_args(p);
-    v.q = q;
-    v.apply_bc = bc;
-    v.psi = psi;
-    v.gbar = dq_bar;
-    v.params = params;
-    v.direct = p->S2;
-    v.rhs = p->XB;
-    if (!e) e = cudaMemsetAsync(p->XB, 0, (size_t)p->xplane * sizeof(float), s);
-    if (!e) e = timed(p, QG_K_STENCIL, s, [&] { return launch_vjp_stencil(v, s); });
-    if (!e) e = timed(p, QG_K_PREP, s, [&] { return launch_vjp_operand(v, nullptr, s); });
-    if (!e) e = run_inversion(p, s);  // the adjoint solve: the inversion is self-adjoint
-    if (!e) e = timed(p, QG_K_OTHER, s, [&] { return launch_vjp_finish(v, p->XC, q_bar, nullptr, s); });
-    return e;
+    // stencil transposes: direct cotangent into S2, the adjoint solve's operand into XA
+    *v = vjp_args(p);
+    v->q = q;
+    v->apply_bc = bc;
+    v->psi = psi;
+    v->gbar = dq_bar;
+    v->params = params;
+    v->direct = p->S2;
+    if (!e) e = timed(p, QG_K_STENCIL, s, [&] { return launch_vjp_stencil(*v, s); });
+    return e ? e : run_inversion(p, s);  // the adjoint solve: the inversion is self-adjoint
 }
 }  // namespace
 
@@ -1667,7 +1659,9 @@ int qg_rhs_vjp(qg_plan* p, const float* q, const float* params, const float* dq_
     cudaStream_t s = (cudaStream_t)stream;
     const int bc = (flags & QG_RHS_APPLY_BC) ? 1 : 0;
     cudaError_t e = cudaMemsetAsync(p->vjp_acc, 0, (size_t)p->n_members * QG_NPARAMS * sizeof(double), s);
-    if (!e) e = rhs_vjp_core(p, q, params, dq_bar, q_bar, bc, s);
+    VjpArgs v;
+    if (!e) e = rhs_vjp_core(p, q, params, dq_bar, bc, s, nullptr, &v);
+    if (!e) e = timed(p, QG_K_OTHER, s, [&] { return launch_vjp_finish(v, p->XC, q_bar, s); });
     if (!e && params_bar) e = launch_vjp_params_only(vjp_args(p), params_bar, s);
     return cuda_err(e);
 }
@@ -1675,7 +1669,7 @@ int qg_rhs_vjp(qg_plan* p, const float* q, const float* params, const float* dq_
 int64_t qg_step_vjp_workspace(const qg_plan* p, int scheme) {
     const Tableau* tb = swm_tableau(scheme);
     if (!p || !tb) return -1;
-    return (int64_t)(4 * tb->n - 2) * p->state_size;
+    return (int64_t)(4 * tb->n - 3) * p->state_size;
 }
 
 namespace {
@@ -1685,9 +1679,8 @@ cudaError_t step_vjp_body(qg_plan* p, const float* y0, const float* params, doub
     const int ns = tb->n;
     const int64_t n = p->state_size;
     // work: stage inputs Y_1 .. Y_{ns-1}, stage derivatives k_0 .. k_{ns-2}, their cotangents
-    // kbar_0 .. kbar_{ns-1}, one stage-input cotangent Ybar, and the layer psi of the stage
-    // inputs Y_0 .. Y_{ns-2} (from the recomputation, so that the reverse sweep inverts only
-    // the last stage's input again)
+    // kbar_0 .. kbar_{ns-1}, and the layer psi of the stage inputs Y_0 .. Y_{ns-2} (from the
+    // recomputation, so that the reverse sweep inverts only the last stage's input again)
     const float* Y[kMaxButcher];
     float* K[kMaxButcher];
     float* kbar[kMaxButcher];
@@ -1696,8 +1689,7 @@ cudaError_t step_vjp_body(qg_plan* p, const float* y0, const float* params, doub
     for (int i = 1; i < ns; ++i) Y[i] = work + (int64_t)(i - 1) * n;
     for (int i = 0; i < ns - 1; ++i) K[i] = work + (int64_t)(ns - 1 + i) * n;
     for (int i = 0; i < ns; ++i) kbar[i] = work + (int64_t)(2 * ns - 2 + i) * n;
-    float* Yb = work + (int64_t)(3 * ns - 2) * n;
-    for (int i = 0; i < ns - 1; ++i) Psi[i] = work + (int64_t)(3 * ns - 1 + i) * n;
+    for (int i = 0; i < ns - 1; ++i) Psi[i] = work + (int64_t)(3 * ns - 2 + i) * n;
     // the step's stage inputs again: Y_s = y0 + dt sum_j a_sj k_j, k_j = F(B(Y_j))
     cudaError_t e = cudaSuccess;
     for (int st = 1; st < ns && !e; ++st) {
@@ -1710,21 +1702,22 @@ cudaError_t step_vjp_body(qg_plan* p, const float* y0, const float* params, doub
             });
         float c[kMaxButcher];
         for (int j = 0; j < st; ++j) c[j] = (float)(dt * tb->a[st][j]);
-        if (!e) e = launch_lincomb(const_cast<float*>(Y[st]), y0, K, c, st, n, s);
+        if (!e) e = launch_lincomb(const_cast<float*>(Y[st]), y0, K, c, st, n, s, use_pdl(p));
     }
     // reverse sweep: kbar_s = dt b_s g; per stage from the last, Ybar = F_vjp(Y_s; kbar_s),
     // then y_bar += Ybar and kbar_j += dt a_sj Ybar (j < s)
     if (!e) {
         float c[kMaxButcher];
         for (int j = 0; j < ns; ++j) c[j] = (float)(dt * tb->b[j]);
-        e = launch_fanout(y_bar, kbar, c, ns, n, s);
+        e = launch_fanout(y_bar, kbar, c, ns, n, p->vjp_acc, p->n_members * QG_NPARAMS, s, use_pdl(p));
     }
-    if (!e) e = cudaMemsetAsync(p->vjp_acc, 0, (size_t)p->n_members * QG_NPARAMS * sizeof(double), s);
     for (int st = ns - 1; st >= 0 && !e; --st) {
-        e = rhs_vjp_core(p, Y[st], params, kbar[st], Yb, 1, s, st < ns - 1 ? Psi[st] : nullptr);
+        VjpArgs v;
+        e = rhs_vjp_core(p, Y[st], params, kbar[st], 1, s, st < ns - 1 ? Psi[st] : nullptr, &v);
         float c[kMaxButcher];
         for (int j = 0; j < st; ++j) c[j] = (float)(dt * tb->a[st][j]);
-        if (!e) e = launch_scatter_bar(y_bar, Yb, kbar, c, st, n, s);
+        if (!e)
+            e = timed(p, QG_K_OTHER, s, [&] { return launch_vjp_scatter(v, p->XC, y_bar, kbar, c, st, s); });
     }
     if (!e && params_bar) e = launch_vjp_params_only(vjp_args(p), params_bar, s);
     return e;
@@ -1778,7 +1771,7 @@ int qg_invert_vjp(qg_plan* p, const float* psi_bar, float* q_bar, void* stream) 
     VjpArgs v = vjp_args(p);
     cudaError_t e = timed(p, QG_K_PREP, s, [&] { return launch_vjp_operand(v, psi_bar, s); });
     if (!e) e = run_inversion(p, s);  // self-adjoint, masked members included
-    if (!e) e = timed(p, QG_K_OTHER, s, [&] { return launch_vjp_finish(v, p->XC, q_bar, nullptr, s); });
+    if (!e) e = timed(p, QG_K_OTHER, s, [&] { return launch_vjp_finish(v, p->XC, q_bar, s); });
     return cuda_err(e);
 }
 
