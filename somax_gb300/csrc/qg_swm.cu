@@ -347,8 +347,7 @@ __device__ __forceinline__ void stage_tile(StageTables& t, const SwmDev& d, cons
 }
 
 template <int NS, bool LAST, bool SAVE>
-__global__ void __launch_bounds__(kSwTX * kSwTY) k_swm_stage(SwmDev d, StageArgs a) {
-    __shared__ StageTables t;
+__device__ __forceinline__ void swm_stage(StageTables& t, const SwmDev& d, const StageArgs& a) {
     const int i0 = blockIdx.x * kSwTX - 1, j0 = blockIdx.y * kSwTY - 1;
     const bool interior = i0 >= 1 && i0 + kStX - 1 <= d.Nx - 3 && j0 >= 1 && j0 + kStY - 1 <= d.Ny - 3;
     if (interior)
@@ -356,6 +355,22 @@ __global__ void __launch_bounds__(kSwTX * kSwTY) k_swm_stage(SwmDev d, StageArgs
     else
         stage_tile<NS, LAST, SAVE, false>(t, d, a);
 }
+
+template <int NS, bool LAST, bool SAVE>
+__global__ void __launch_bounds__(kSwTX * kSwTY) k_swm_stage(SwmDev d, StageArgs a) {
+    __shared__ StageTables t;
+    swm_stage<NS, LAST, SAVE>(t, d, a);
+}
+
+// The same held to 64 registers, four CTAs an SM: on basins of many waves the latency of the loads
+// bounds a stage (the last of Tsit5 took 128 registers, two CTAs an SM).  Tsit5 at 1024 x 1024 x 3: 66.6 -> 62.2 us a stage; 700 x 1000 x 2: 30.7 -> 29.2; 512 x 512 x 3: 18.9 ->
+// 19.4, so that it takes over from kTightCtas CTAs up, where the spilled registers are worth it.
+template <int NS, bool LAST>
+__global__ void __launch_bounds__(kSwTX * kSwTY, 4) k_swm_stage_tight(SwmDev d, StageArgs a) {
+    __shared__ StageTables t;
+    swm_stage<NS, LAST, false>(t, d, a);
+}
+constexpr unsigned kTightCtas = 1824;  // twelve an SM
 
 // ---- cluster-resident engine: every step of a small basin in one thread-block cluster -----
 //
@@ -1067,8 +1082,13 @@ cudaError_t launch_ns(const qg_swm_plan* p, const StageArgs& a, cudaStream_t s) 
         else
             k_swm_stage<NS, false, true><<<g, b, 0, s>>>(p->d, a);
     } else {
-        if (a.last)
+        const bool tight = g.x * g.y >= kTightCtas;
+        if (NS >= 2 && tight && a.last)
+            k_swm_stage_tight<NS, true><<<g, b, 0, s>>>(p->d, a);
+        else if (a.last)
             k_swm_stage<NS, true, false><<<g, b, 0, s>>>(p->d, a);
+        else if (NS >= 3 && tight)
+            k_swm_stage_tight<NS, false><<<g, b, 0, s>>>(p->d, a);
         else
             k_swm_stage<NS, false, false><<<g, b, 0, s>>>(p->d, a);
     }
