@@ -53,12 +53,6 @@ __device__ __forceinline__ int64_t xidx(const MemberDev& M, int l, int j, int i)
     return M.off_x + ((int64_t)l * M.Ny + j) * M.Px + i;
 }
 
-template <typename T>
-__device__ __forceinline__ T warp_sum(T v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    return v;
-}
-
 }  // namespace
 
 // Stencil part of the RHS VJP: one 32 x 4 tile, every layer, per CTA (128 threads a layer).  Writes
@@ -127,8 +121,7 @@ __global__ void __launch_bounds__(kTileThreads* kMaxLayers)
     const int j = jt + c / TX, i = it + c % TX, e = (c / TX + HB) * SX + c % TX + HB;
     const bool cell = on && j < Ny && i < Nx;
     const bool ring = cell && G.ring(j, i), land = cell && G.land(j, i);
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    float pb = 0.f;
+    float pb = 0.f, lq = 0.f, lp = 0.f, wind = 0.f;  // of cells that the parameters' terms read
     if (cell) {
         // A(dj, di): a at b + d;  F / Q(cj, ci, dj, di): psi / qb at b + c + d
         auto A = [&](int dj, int di) { return sa[e + dj * SX + di]; };
@@ -166,25 +159,25 @@ __global__ void __launch_bounds__(kTileThreads* kMaxLayers)
         if (l == nl - 1) pb -= kappa * lfa;
         if ((ring && !M.barotropic) || land) pb = 0.f;
         if (!ring) {
-            const float lq = (Q(0, 0, 0, 1) - 2.f * Q(0, 0, 0, 0) + Q(0, 0, 0, -1)) * idx2 +
-                             (Q(0, 0, 1, 0) - 2.f * Q(0, 0, 0, 0) + Q(0, 0, -1, 0)) * idy2;
-            acc[QG_P_NU] = (double)A(0, 0) * lq;
-            acc[QG_P_NU4] = -(double)sm[e] * lq;  // -<a, lap(M lap qb)> = -<M Lf(a), lap qb>
-            if (l == nl - 1) {
-                const float lp = (F(0, 0, 0, 1) - 2.f * F(0, 0, 0, 0) + F(0, 0, 0, -1)) * idx2 +
-                                 (F(0, 0, 1, 0) - 2.f * F(0, 0, 0, 0) + F(0, 0, -1, 0)) * idy2;
-                acc[QG_P_KAPPA] = -(double)A(0, 0) * lp;
-            }
+            lq = (Q(0, 0, 0, 1) - 2.f * Q(0, 0, 0, 0) + Q(0, 0, 0, -1)) * idx2 +
+                 (Q(0, 0, 1, 0) - 2.f * Q(0, 0, 0, 0) + Q(0, 0, -1, 0)) * idy2;
+            lp = (F(0, 0, 0, 1) - 2.f * F(0, 0, 0, 0) + F(0, 0, 0, -1)) * idx2 +
+                 (F(0, 0, 1, 0) - 2.f * F(0, 0, 0, 0) + F(0, 0, -1, 0)) * idy2;
         }
         // the wind: every cell of layer 0, ring included; dq = 0 on land
-        if (l == 0 && !land) acc[QG_P_TAU0] = (double)gbar[G.c(j, i)] * M.F[j] * M.invH0;
+        if (l == 0 && !land) wind = gbar[G.c(j, i)];
     }
     if (on) spb[l * kTileThreads + c] = pb;
+    // the cotangents: a lap q, -(M Lf(a)) lap q, [bottom] -a lap psi, [top] g F / H0 (a warp is a row)
+    const float a0 = cell ? sa[e] : 0.f;
+    double sum[4];
+    sum[QG_P_NU] = warp_dot(a0, lq);
+    sum[QG_P_NU4] = -warp_dot(cell ? sm[e] : 0.f, lq);
+    sum[QG_P_KAPPA] = l == nl - 1 ? -warp_dot(a0, lp) : 0.0;
+    sum[QG_P_TAU0] = l == 0 ? warp_dot(wind, cell ? M.F[j] : 0.f) * M.invH0 : 0.0;
+    if ((threadIdx.x & 31) == 0)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        acc[k] = warp_sum(acc[k]);
-        if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = acc[k];
-    }
+        for (int k = 0; k < 4; ++k) red[k][threadIdx.x >> 5] = sum[k];
     __syncthreads();
     if (cell) {
         float v = 0.f;

@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(kVjX * kVjY) k_swm_vjp(SwmDev d, const float* 
     const float nu = params[0], kappa = params[1];
     const int tx = tid % kVjX, ty = tid / kVjX, e = (ty + 2) * S + tx + 2;
     const int b = i0 + 2 + tx, a = j0 + 2 + ty;
-    double pnu = 0.0, pkap = 0.0, ptau = 0.0;
+    float pnu = 0.f, pkap = 0.f, ptau = 0.f;
     if (b < d.Nx && a < d.Ny) {
         const int64_t o = (int64_t)a * d.Nx + b;
         // the potential's cotangents of the layers below, then this one's
@@ -745,31 +745,27 @@ __global__ void __launch_bounds__(kVjX * kVjY) k_swm_vjp(SwmDev d, const float* 
         if (in) {
             const float lu = (su[e + 1] - 2.f * u0 + su[e - 1]) * d.idx2 + (su[e + S] - 2.f * u0 + su[e - S]) * d.idy2;
             const float lv = (sv[e + 1] - 2.f * v0 + sv[e - 1]) * d.idx2 + (sv[e + S] - 2.f * v0 + sv[e - S]) * d.idy2;
-            pnu = (double)(gu[e] * lu + gv[e] * lv);
+            pnu = gu[e] * lu + gv[e] * lv;
         }
         // drag (bottom layer, every cell) and wind (top layer, every cell)
         const float guo = gbar[field + lo + o], gvo = gbar[2 * field + lo + o];
         if (k == d.nl - 1) {
             ub -= kappa * guo;
             vb -= kappa * gvo;
-            pkap = -(double)(guo * u0 + gvo * v0);
+            pkap = -(guo * u0 + gvo * v0);
         }
-        if (k == 0) ptau = (double)(guo * __ldg(d.wx + a) * d.invH0);
+        if (k == 0) ptau = guo * __ldg(d.wx + a) * d.invH0;
         hb += __ldg(d.gp + k) * pcum;
         ybar[lo + o] = hb;
         ybar[field + lo + o] = ub;
         ybar[2 * field + lo + o] = vb;
     }
     // parameter cotangents: one double atomic a CTA
-    for (int m = 16; m > 0; m >>= 1) {
-        pnu += __shfl_down_sync(0xffffffffu, pnu, m);
-        pkap += __shfl_down_sync(0xffffffffu, pkap, m);
-        ptau += __shfl_down_sync(0xffffffffu, ptau, m);
-    }
+    const double snu = warp_total(pnu), skap = k == d.nl - 1 ? warp_total(pkap) : 0.0, stau = k == 0 ? warp_total(ptau) : 0.0;
     if ((tid & 31) == 0) {
-        red[0][tid >> 5] = pnu;
-        red[1][tid >> 5] = pkap;
-        red[2][tid >> 5] = ptau;
+        red[0][tid >> 5] = snu;
+        red[1][tid >> 5] = skap;
+        red[2][tid >> 5] = stau;
     }
     __syncthreads();
     if (tid < 3) {
