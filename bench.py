@@ -433,7 +433,8 @@ SWM_GRAD_DESC = ("swm_grad_jet64: one gradient per bench step of the misfit 0.5 
 
 
 def swm_grad_launches(engine: str, n_steps: int, every: int, ns: int = 6) -> int:
-    """Kernel launches of one Tsit5 gradient: the forward (boundary rules, then a call per
+    """Kernel launches of one Tsit5 gradient step by step with a kernel for every update (the count
+    that the fused ones are held against): the forward (boundary rules, then a call per
     checkpoint segment), the backward's recomputation (a one-step call per step of a segment
     but its first), one qg_swm_step_vjp per step (ns - 1 stage and combine launches, ns
     cotangent initialisations, per stage the three VJP kernels and the y_bar update, one update
@@ -444,6 +445,17 @@ def swm_grad_launches(engine: str, n_steps: int, every: int, ns: int = 6) -> int
     recompute = (n_steps - segs) * (1 if per_call else ns)
     vjp = 2 * (ns - 1) + ns + 4 * ns + ns * (ns - 1) // 2 + 1
     return fwd + recompute + n_steps * vjp + 1
+
+
+def swm_segment_launches(engine: str, n_steps: int, every: int, ns: int = 6) -> int:
+    """Kernel launches of one Tsit5 gradient whose reverse sweep runs by segments: the forward
+    (boundary rules, then a call per checkpoint segment), the backward's segments (every step's
+    stages once, the last step's last one as a combination; zeroed sums; per step the stage
+    cotangents and per stage the VJP and its scatter; the parameter write-out) and the final
+    transposed boundary rules."""
+    segs = -(-n_steps // every)
+    fwd = 1 + (segs if engine == "cluster" else n_steps * ns)
+    return fwd + n_steps * ns + 2 * segs + n_steps * (1 + 2 * ns) + 1
 
 
 def run_swm_grad(args, dev, world, rank, local):
@@ -506,7 +518,7 @@ def run_swm_grad(args, dev, world, rank, local):
         "config": {"workload": SWM_GRAD_DESC, "engine": m.plan(dev).engine(cfg.scheme)},
         "e2e": {"value": world * args.steps * days / e2e_s, "unit": UNIT, "h2d_bytes_per_step": hh.numel() * 4,
                 "d2h_bytes_per_step": out.numel() * 4, "api": "MultilayerShallowWater2D.integrate + autograd"},
-        "gpu_launches": args.steps * swm_grad_launches(m.plan(dev).engine(cfg.scheme)["engine"], n_steps, every),
+        "gpu_launches": args.steps * swm_segment_launches(m.plan(dev).engine(cfg.scheme)["engine"], n_steps, every),
         "clocks": clk.summary(),
     }
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
@@ -745,7 +757,7 @@ def traffic_table():
         return json.load(f).get("bytes_per_launch", {})
 
 
-def roofline(W, stats, precision, name, cluster=False, step_ms=None):
+def roofline(W, stats, precision, name, cluster=False, step_ms=None, rows=False):
     """Roofline of every kernel class from the profiled pass's per-launch event times.
 
     The profiled pass runs one bench step with CUDA events around every launch (graphs and
@@ -762,6 +774,9 @@ def roofline(W, stats, precision, name, cluster=False, step_ms=None):
       cluster      the cluster-resident step kernel (class 4 when the plan steps with it): the
                    state in (4 B) and out (4 B) once per launch; everything else lives in shared
                    memory, so the kernel is bound by its SMs' FP32 work and barriers, not HBM
+    The row engine's kernels (``rows``) fall into the same classes with the same bytes: its column
+    kernel (both y transforms) into dst_gemm, its row kernel into rhs_stencil; they run on the FP32
+    cores, so that no tensor figure applies.
     Issued tensor flops of a DST-I pass: 2 N per element (three products for BF16x3).  A
     kernel is HBM-bound when its bytes / peak bandwidth exceed its flops / peak throughput.
     The dominant class (largest total time) is the headline."""
@@ -770,8 +785,8 @@ def roofline(W, stats, precision, name, cluster=False, step_ms=None):
     bytes_per = {0: 12.0 * lc, 1: 8.0 * lc, 2: 20.0 * lc, 3: 8.0 * lc}
     if cluster:
         bytes_per[4] = 8.0 * lc
-    flops_per = {1: W.gemm_flops_per_pass() * (3.0 if precision == "bf16x3" else 1.0)}
-    traffic = traffic_table().get(name, {})
+    flops_per = {} if rows else {1: W.gemm_flops_per_pass() * (3.0 if precision == "bf16x3" else 1.0)}
+    traffic = {} if rows else traffic_table().get(name, {})  # measured on the pass-by-pass kernels
     prof_total = sum(ms for ms, n in stats.values() if n)
     scale = step_ms / prof_total if step_ms and prof_total > 0 else 1.0
     kernels = {}
@@ -1016,7 +1031,8 @@ def main():
         launches_per_day = sum(n for _, n in stats.values())  # every launch of one gradient, counted
     else:
         launches_per_day = plan.launches_per_call(W.steps_per_day, W.scheme)
-    roof = roofline(W, stats, args.precision, args.config, plan.engine()["cluster_ctas"] > 0, ms_per_step)
+    roof = roofline(W, stats, args.precision, args.config, plan.engine()["cluster_ctas"] > 0, ms_per_step,
+                    bool(plan.engine().get("rows")))
 
     # ---- the plain FP32 single-member path on the same members (the metric's baseline) ----
     vs_baseline, plain = None, None

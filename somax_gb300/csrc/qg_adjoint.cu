@@ -31,6 +31,7 @@
 
 #include "qg_internal.cuh"
 #include "qg_stencil_tile.cuh"
+#include "qg_warp.cuh"
 
 namespace qg {
 

@@ -35,6 +35,7 @@
 
 #include "qg_device.cuh"
 #include "qg_internal.cuh"
+#include "qg_warp.cuh"
 
 namespace qg {
 namespace {

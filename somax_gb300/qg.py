@@ -426,10 +426,10 @@ class Plan:
             stencil = len({m.n_layers for m in self.members})
         else:
             stencil = 1
-        solve = 4 * (1 + self.refine) + self.refine
-        inversion = solve
-        if masked:  # capacitance correction(s), each followed by a solve
-            inversion += (1 + self.refine) * (1 + (1 if self.refine else 0) + solve)
+        inversion = 4 * (1 + self.refine) + self.refine
+        if masked:  # a solve, then per sweep the capacitance correction, the residual and a solve
+            sweeps = 1 if self.refine == 0 else 5 if self.precision == "tf32" else 3
+            inversion = 4 + sweeps * (1 + (1 if self.refine else 0) + 4)
         per_stage = inversion + stencil + (1 if butcher else 0)
         return 2 + n_steps * stages * per_stage
 
