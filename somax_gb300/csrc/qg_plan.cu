@@ -894,15 +894,23 @@ cudaError_t autotune_stencil(qg_plan* p) {
             e = run_dst_solve(p, s);
             if (!e) e = launch_stencil(p, a, s, false);
         }
-        if (!e) e = cudaEventRecord(e0, s);
-        for (int rep = 0; rep < 3 && !e; ++rep) {
-            e = run_dst_solve(p, s);
-            if (!e) e = launch_stencil(p, a, s, false);
-        }
-        if (!e) e = cudaEventRecord(e1, s);
-        if (!e) e = cudaEventSynchronize(e1);
-        if (!e) e = cudaEventElapsedTime(&ms, e0, e1);
-        p->tune_ms[v] = ms / 3.f;
+        auto timed_stages = [&](int n) {
+            if (!e) e = cudaEventRecord(e0, s);
+            for (int rep = 0; rep < n && !e; ++rep) {
+                e = run_dst_solve(p, s);
+                if (!e) e = launch_stencil(p, a, s, false);
+            }
+            if (!e) e = cudaEventRecord(e1, s);
+            if (!e) e = cudaEventSynchronize(e1);
+            if (!e) e = cudaEventElapsedTime(&ms, e0, e1);
+            p->tune_ms[v] = ms / n;
+        };
+        // one stage, and three if it takes less than 1.5 times the best so far: the slow variants of a
+        // size would take most of the tuning's time
+        timed_stages(1);
+        float best = ms;
+        for (int u = 0; u < v; ++u) best = std::min(best, p->tune_ms[u]);
+        if (ms < 1.5f * best) timed_stages(3);
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);

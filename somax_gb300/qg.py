@@ -10,6 +10,7 @@ barotropic model), ``Ny = ny + 2``, ``Nx = nx + 2``.
 
 from __future__ import annotations
 
+import array
 import ctypes as C
 import dataclasses
 import math
@@ -187,8 +188,8 @@ def _device_vector(vals, device) -> torch.Tensor:
     device = torch.device("cpu" if device is None else device)
     if device.type != "cuda" or device.index not in (None, torch.cuda.current_device()):
         return torch.tensor(vals, dtype=torch.float32).to(device)
-    out = torch.empty(len(vals), dtype=torch.float32, device=device)
-    check(_lib.lib().qg_write(C.c_void_p(out.data_ptr()), (C.c_float * len(vals))(*vals), len(vals),
+    out, host = torch.empty(len(vals), dtype=torch.float32, device=device), array.array("f", vals)
+    check(_lib.lib().qg_write(C.c_void_p(out.data_ptr()), C.c_void_p(host.buffer_info()[0]), len(vals),
                               _stream_handle(out.device)), "qg_write")
     return out
 
