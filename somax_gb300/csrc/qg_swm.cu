@@ -603,8 +603,8 @@ __global__ void __launch_bounds__(kScThreads) k_swm_cluster(SwmClusterArgs a) {
 // Bound: launches and latency on small basins.  Two kernels that formed every intermediate from
 // global memory at each of its readers (~200 loads a point and layer, boundary rules and all), a
 // third for the boundary rules and an axpy per stage derivative took 331 us for a Tsit5 step's
-// adjoint at 2 x 66^2, 63 launches; these take 123 us, the forward stages included (the smallest
-// tile that fills a warp's row: 18 CTAs a layer).
+// adjoint at 2 x 66^2, 63 launches; these take 94 us, the forward stages included (32 x 4 is the
+// smallest tile of whole warps' rows: 51 CTAs a layer).
 
 constexpr int kVjX = 32, kVjY = 4, kVjSX = kVjX + 4, kVjSY = kVjY + 4, kVjE = kVjSX * kVjSY;
 
