@@ -864,7 +864,8 @@ def plain_fp32_rate(dev, mix, repeats: int = 3):
             raise RuntimeError(f"plain FP32 path flagged a device error on {cfg.name}")
         ms = statistics.median(ts)
         per_class[cfg.name] = {"members": count, "ms_per_model_day": ms,
-                               "engine": "cluster" if plan.engine()["cluster_ctas"] else "multi-launch",
+                               "engine": ("cluster" if plan.engine()["cluster_ctas"] else
+                                          "rows" if plan.engine()["rows"] else "multi-launch"),
                                "stencil": plan.tuning()["stencil"]}
         t_day += count * ms
         total += count

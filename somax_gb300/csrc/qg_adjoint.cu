@@ -98,7 +98,17 @@ __global__ void __launch_bounds__(kTileThreads* kMaxLayers)
     const float nu = P[QG_P_NU], kappa = P[QG_P_KAPPA], nu4 = P[QG_P_NU4];
     const float idx2 = M.inv_dx2, idy2 = M.inv_dy2, i12 = M.inv_12dxdy, b12 = M.beta_12dx;
     const int j0 = jt - HB, i0 = it - HB;
-    if (on)
+    // the tile and its halo strictly inside a member without land: no rules to apply
+    const bool inner = !G.mask && j0 >= 1 && i0 >= 1 && j0 + SY < Ny && i0 + SX < Nx;
+    if (on && inner) {
+        const int64_t o0 = G.c(j0, i0) + l * G.lc;
+        for (int k = c; k < kBox; k += kTileThreads) {
+            const int64_t o = o0 + (k / SX) * Nx + k % SX;
+            sa[k] = gbar[o];
+            sq[k] = q[o];
+            sp[k] = psi[o];
+        }
+    } else if (on)
         for (int k = c; k < kBox; k += kTileThreads) {
             const int j = j0 + k / SX, i = i0 + k % SX;
             const bool in = j >= 0 && j < Ny && i >= 0 && i < Nx;
@@ -114,7 +124,7 @@ __global__ void __launch_bounds__(kTileThreads* kMaxLayers)
         for (int k = c; k < kBox; k += kTileThreads) {
             const int y = k / SX, x = k % SX, j = j0 + y, i = i0 + x;
             float v = 0.f;  // lap(qb) is zero on the ring and on land
-            if (y > 0 && x > 0 && y < SY - 1 && x < SX - 1 && interior(j, i, Ny, Nx) && !G.land(j, i))
+            if (y > 0 && x > 0 && y < SY - 1 && x < SX - 1 && (inner || (interior(j, i, Ny, Nx) && !G.land(j, i))))
                 v = (sa[k + 1] - 2.f * sa[k] + sa[k - 1]) * idx2 + (sa[k + SX] - 2.f * sa[k] + sa[k - SX]) * idy2;
             sm[k] = v;
         }
@@ -162,8 +172,9 @@ __global__ void __launch_bounds__(kTileThreads* kMaxLayers)
         if (!ring) {
             lq = (Q(0, 0, 0, 1) - 2.f * Q(0, 0, 0, 0) + Q(0, 0, 0, -1)) * idx2 +
                  (Q(0, 0, 1, 0) - 2.f * Q(0, 0, 0, 0) + Q(0, 0, -1, 0)) * idy2;
-            lp = (F(0, 0, 0, 1) - 2.f * F(0, 0, 0, 0) + F(0, 0, 0, -1)) * idx2 +
-                 (F(0, 0, 1, 0) - 2.f * F(0, 0, 0, 0) + F(0, 0, -1, 0)) * idy2;
+            if (l == nl - 1)
+                lp = (F(0, 0, 0, 1) - 2.f * F(0, 0, 0, 0) + F(0, 0, 0, -1)) * idx2 +
+                     (F(0, 0, 1, 0) - 2.f * F(0, 0, 0, 0) + F(0, 0, -1, 0)) * idy2;
         }
         // the wind: every cell of layer 0, ring included; dq = 0 on land
         if (l == 0 && !land) wind = gbar[G.c(j, i)];

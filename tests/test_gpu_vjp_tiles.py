@@ -20,7 +20,7 @@ P = dict(lateral_viscosity=PHYS["nu"], bottom_drag=PHYS["kappa"], wind_amplitude
 
 
 @pytest.mark.parametrize("apply_bc", [False, True])
-@pytest.mark.parametrize("sizes", [[(29, 2, 1)], [(30, 3, 2)], [(31, 6, 3)], [(62, 4, 2)], [(5, 15, 4)], [(3, 14, 8)],
+@pytest.mark.parametrize("sizes", [[(29, 2, 1)], [(30, 3, 2)], [(31, 6, 3)], [(62, 4, 2)], [(5, 15, 4)], [(3, 14, 8)], [(70, 9, 2)],
                                    [(30, 6, 1), (4, 9, 6), (33, 2, 3)]])
 def test_rhs_vjp_at_tile_edges(sizes, apply_bc):
     os_, specs, qs, gs = [], [], [], []
