@@ -182,14 +182,11 @@ __global__ void __launch_bounds__(kTileThreads* kMaxLayers)
     if (on) spb[l * kTileThreads + c] = pb;
     // the cotangents: a lap q, -(M Lf(a)) lap q, [bottom] -a lap psi, [top] g F / H0 (a warp is a row)
     const float a0 = cell ? sa[e] : 0.f;
-    double sum[4];
-    sum[QG_P_NU] = warp_dot(a0, lq);
-    sum[QG_P_NU4] = -warp_dot(cell ? sm[e] : 0.f, lq);
-    sum[QG_P_KAPPA] = l == nl - 1 ? -warp_dot(a0, lp) : 0.0;
-    sum[QG_P_TAU0] = l == 0 ? warp_dot(wind, cell ? M.F[j] : 0.f) * M.invH0 : 0.0;
-    if ((threadIdx.x & 31) == 0)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) red[k][threadIdx.x >> 5] = sum[k];
+    static_assert(QG_P_NU == 0 && QG_P_KAPPA == 1 && QG_P_TAU0 == 2 && QG_P_NU4 == 3, "the order of the sums");
+    const double sum = warp_sum4((double)a0 * lq, l == nl - 1 ? -(double)a0 * lp : 0.0,
+                                 l == 0 ? (double)wind * (cell ? M.F[j] : 0.f) * M.invH0 : 0.0,
+                                 -(double)(cell ? sm[e] : 0.f) * lq);
+    if ((threadIdx.x & 31) < 4) red[threadIdx.x & 31][threadIdx.x >> 5] = sum;
     __syncthreads();
     if (cell) {
         float v = 0.f;

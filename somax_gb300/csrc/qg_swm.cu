@@ -762,12 +762,8 @@ __global__ void __launch_bounds__(kVjX * kVjY) k_swm_vjp(SwmDev d, const float* 
         ybar[2 * field + lo + o] = vb;
     }
     // parameter cotangents: one double atomic a CTA
-    const double snu = warp_total(pnu), skap = k == d.nl - 1 ? warp_total(pkap) : 0.0, stau = k == 0 ? warp_total(ptau) : 0.0;
-    if ((tid & 31) == 0) {
-        red[0][tid >> 5] = snu;
-        red[1][tid >> 5] = skap;
-        red[2][tid >> 5] = stau;
-    }
+    const double sum = warp_sum4(pnu, pkap, ptau, 0.0);  // pkap and ptau are 0 away from their layer
+    if ((tid & 31) < 3) red[tid & 31][tid >> 5] = sum;
     __syncthreads();
     if (tid < 3) {
         double v = 0.0;

@@ -3,40 +3,23 @@
 
 namespace qg {
 
-// Sums over a warp for FP64 accumulators without the FP64 units (two lanes a clock an SM; a warp of an
-// adjoint kernel spent 30 of their instructions, the gradient of 20 steps at 256 x 256 x 3 took 9.30 ms
-// with them, 9.13 without).  Pairs of floats carry what a float sum rounds off, 45 bits of the largest
-// term and more; operands of a product are scaled by powers of two so that none under- or overflows.
-// Infinities and NaN take the FP64 sum.
-__device__ __forceinline__ double warp_sum_pair(float h, float l) {
+// Sums over a warp of four FP64 values at once: lane l gets the total of value l % 4.  FP64 throughout
+// (parameter cotangents cancel over the basin, and their terms spread over the whole FP32 range).  The
+// first two rounds halve the values a lane holds, so that the four take 6 additions a lane and not 20:
+// the FP64 units serve two lanes a clock an SM.  The gradient of 20 steps at 256 x 256 x 3 takes 9.03 ms;
+// with a sum for each value 9.30; with products and sums in pairs of FP32 numbers, which lose bits of
+// products far below the operands' largest values, 9.07.
+__device__ __forceinline__ double warp_sum4(double a, double b, double c, double d) {
+    const int lane = threadIdx.x & 31;
+    const bool odd = lane & 1, high = lane & 2;
+    double ab = odd ? b : a, cd = odd ? d : c;
+    ab += __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
+    cd += __shfl_xor_sync(0xffffffffu, odd ? c : d, 1);
+    double v = high ? cd : ab;
+    v += __shfl_xor_sync(0xffffffffu, high ? ab : cd, 2);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float h2 = __shfl_xor_sync(0xffffffffu, h, o), l2 = __shfl_xor_sync(0xffffffffu, l, o);
-        const float s = h + h2, b = s - h;
-        l += l2 + ((h - (s - b)) + (h2 - b));
-        h = s;
-    }
-    return (double)h + (double)l;
-}
-__device__ __forceinline__ double warp_sum_f64(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    for (int o = 4; o < 32; o *= 2) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
-}
-// the sum of v over the warp's lanes, in every lane
-__device__ __forceinline__ double warp_total(float v) {
-    const unsigned e = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(v))) >> 23;
-    return e >= 249 ? warp_sum_f64((double)v) : warp_sum_pair(v, 0.f);  // 32 terms stay below 2^127
-}
-// the sum of a * b over the warp's lanes, in every lane
-__device__ __forceinline__ double warp_dot(float a, float b) {
-    const unsigned ea = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(a))) >> 23;
-    const unsigned eb = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(b))) >> 23;
-    if (ea > 253 || eb > 253) return warp_sum_f64((double)a * (double)b);
-    // the largest of each below 2: 2^(127 - e)
-    const float x = a * __uint_as_float((254 - ea) << 23), y = b * __uint_as_float((254 - eb) << 23);
-    const float h = x * y;
-    return warp_sum_pair(h, fmaf(x, y, -h)) * __hiloint2double((int)(ea + eb - 254 + 1023) << 20, 0);
 }
 
 }  // namespace qg
