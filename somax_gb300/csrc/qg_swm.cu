@@ -363,9 +363,12 @@ __global__ void __launch_bounds__(kSwTX * kSwTY) k_swm_stage(SwmDev d, StageArgs
     swm_stage<NS, LAST, SAVE>(t, d, a);
 }
 
-// The same held to 64 registers, four CTAs an SM: on basins of many waves the latency of the loads
-// bounds a stage (the last of Tsit5 took 128 registers, two CTAs an SM).  Tsit5 at 1024 x 1024 x 3: 66.6 -> 62.2 us a stage; 700 x 1000 x 2: 30.7 -> 29.2; 512 x 512 x 3: 18.9 ->
-// 19.4, so that it takes over from kTightCtas CTAs up, where the spilled registers are worth it.
+// The same held to 64 registers, four CTAs an SM, for stages that read three derivatives or more: on
+// basins of many waves the latency of the loads bounds a stage (the last of Tsit5 took 128 registers, two
+// CTAs an SM).  Tsit5 at 1024 x 1024 x 3: 66.6 -> 62.2 us a stage; 700 x 1000 x 2: 30.7 -> 29.2; 512 x 512
+// x 3: 18.9 -> 19.4, so that it takes over from kTightCtas CTAs up, where the spilled registers are worth
+// it.  With two derivatives (SSP-RK3's last stage) they are not: eight steps at 1024 x 1024 x 3 take
+// 1348 us with them and 1270 without, at 700 x 1000 x 2 604 and 579.
 template <int NS, bool LAST>
 __global__ void __launch_bounds__(kSwTX * kSwTY, 4) k_swm_stage_tight(SwmDev d, StageArgs a) {
     __shared__ StageTables t;
@@ -1075,13 +1078,16 @@ cudaError_t launch_ns(const qg_swm_plan* p, const StageArgs& a, cudaStream_t s) 
         else
             k_swm_stage<NS, false, true><<<g, b, 0, s>>>(p->d, a);
     } else {
-        const bool tight = g.x * g.y >= kTightCtas;
-        if (NS >= 2 && tight && a.last)
-            k_swm_stage_tight<NS, true><<<g, b, 0, s>>>(p->d, a);
-        else if (a.last)
+        if constexpr (NS >= 3)
+            if (g.x * g.y >= kTightCtas) {
+                if (a.last)
+                    k_swm_stage_tight<NS, true><<<g, b, 0, s>>>(p->d, a);
+                else
+                    k_swm_stage_tight<NS, false><<<g, b, 0, s>>>(p->d, a);
+                return cudaGetLastError();
+            }
+        if (a.last)
             k_swm_stage<NS, true, false><<<g, b, 0, s>>>(p->d, a);
-        else if (NS >= 3 && tight)
-            k_swm_stage_tight<NS, false><<<g, b, 0, s>>>(p->d, a);
         else
             k_swm_stage<NS, false, false><<<g, b, 0, s>>>(p->d, a);
     }
