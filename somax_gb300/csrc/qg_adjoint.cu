@@ -56,16 +56,20 @@ __device__ __forceinline__ int64_t xidx(const MemberDev& M, int l, int j, int i)
 
 }  // namespace
 
-// Stencil part of the RHS VJP: one 32 x 4 tile, every layer, per CTA (128 threads a layer).  Writes
-// the direct cotangent of qb (x-row plane `direct`), Cm2l^T Z psi_bar as the operand of the adjoint
-// solve (and its FP32 copy for the refinement residual), and accumulates the parameter cotangents into
-// `pacc` (double, QG_NPARAMS per member).
+// Stencil part of the RHS VJP of members of one layer count: one 32 x 4 tile, every layer, per CTA (128
+// threads a layer; blockDim.x = 128 layers).  Writes the direct cotangent of qb (x-row plane `direct`),
+// Cm2l^T Z psi_bar as the operand of the adjoint solve (and its FP32 copy for the refinement residual), and
+// accumulates the parameter cotangents into `pacc` (double, QG_NPARAMS per member).
 //
 // Bound: latency on the sizes a gradient is taken of (200 000 cells make 594 CTAs of 384 threads).  The
 // layers lie side by side so that their mix is a sum over shared memory; a CTA per layer added them
 // up with atomics in a zeroed FP32 plane that another kernel turned into the operand, and a third, of
 // sixteen CTAs, summed the wind's cotangent: 41 us a stage at 256 x 256 x 3.  With the finish's sums and
-// early starts the gradient of 20 steps there takes 9.3 ms, 11.0 before.
+// early starts the gradient of 20 steps there took 9.3 ms, 11.0 before.
+//
+// A plan of mixed layer counts launches once for each, side by side.  With one launch as wide as the
+// deepest member, the CTAs of the others held warps that only waited: a qg_rhs_vjp of 256 members of one,
+// three and five layers took 3071 us (2006 so; 2711 with a CTA per layer), of eight small ones 84 (82).
 constexpr int kTileThreads = TX * TY, kBox = SX * SY;  // cells of a tile, with its halo
 constexpr int kSubX = kTileLX / TX, kSubY = kTileLY / TY;  // CTAs per 64 x 16 tile of the list
 constexpr size_t vjp_stencil_smem(int nl) { return (size_t)nl * (4 * kBox + kTileThreads) * sizeof(float); }
@@ -87,8 +91,7 @@ __global__ void __launch_bounds__(kTileThreads* kMaxLayers)
     const int jt = t.ty * kTileLY + part / kSubX * TY, it = t.tx * kTileLX + part % kSubX * TX;
     if (jt >= Ny || it >= Nx) return;  // all of the CTA
     const int l = threadIdx.x / kTileThreads, c = threadIdx.x % kTileThreads;
-    const bool on = l < nl;
-    float* sa = smem + (size_t)(on ? l : 0) * 4 * kBox;  // a = interior-masked cotangent
+    float* sa = smem + (size_t)l * 4 * kBox;             // a = interior-masked cotangent
     float* sq = sa + kBox;                               // qb
     float* sp = sq + kBox;                               // psi (layer, ring zeroed for the baroclinic model)
     float* sm = sp + kBox;                               // M Lf(a)
@@ -100,7 +103,7 @@ __global__ void __launch_bounds__(kTileThreads* kMaxLayers)
     const int j0 = jt - HB, i0 = it - HB;
     // the tile and its halo strictly inside a member without land: no rules to apply
     const bool inner = !G.mask && j0 >= 1 && i0 >= 1 && j0 + SY < Ny && i0 + SX < Nx;
-    if (on && inner) {
+    if (inner) {
         const int64_t o0 = G.c(j0, i0) + l * G.lc;
         for (int k = c; k < kBox; k += kTileThreads) {
             const int64_t o = o0 + (k / SX) * Nx + k % SX;
@@ -108,7 +111,7 @@ __global__ void __launch_bounds__(kTileThreads* kMaxLayers)
             sq[k] = q[o];
             sp[k] = psi[o];
         }
-    } else if (on)
+    } else {
         for (int k = c; k < kBox; k += kTileThreads) {
             const int j = j0 + k / SX, i = i0 + k % SX;
             const bool in = j >= 0 && j < Ny && i >= 0 && i < Nx;
@@ -119,18 +122,18 @@ __global__ void __launch_bounds__(kTileThreads* kMaxLayers)
             sq[k] = sea && !(apply_bc && ring) ? q[o] : 0.f;
             sp[k] = sea ? psi[o] : 0.f;
         }
+    }
     __syncthreads();
-    if (on)
-        for (int k = c; k < kBox; k += kTileThreads) {
-            const int y = k / SX, x = k % SX, j = j0 + y, i = i0 + x;
-            float v = 0.f;  // lap(qb) is zero on the ring and on land
-            if (y > 0 && x > 0 && y < SY - 1 && x < SX - 1 && (inner || (interior(j, i, Ny, Nx) && !G.land(j, i))))
-                v = (sa[k + 1] - 2.f * sa[k] + sa[k - 1]) * idx2 + (sa[k + SX] - 2.f * sa[k] + sa[k - SX]) * idy2;
-            sm[k] = v;
-        }
+    for (int k = c; k < kBox; k += kTileThreads) {
+        const int y = k / SX, x = k % SX, j = j0 + y, i = i0 + x;
+        float v = 0.f;  // lap(qb) is zero on the ring and on land
+        if (y > 0 && x > 0 && y < SY - 1 && x < SX - 1 && (inner || (interior(j, i, Ny, Nx) && !G.land(j, i))))
+            v = (sa[k + 1] - 2.f * sa[k] + sa[k - 1]) * idx2 + (sa[k + SX] - 2.f * sa[k] + sa[k - SX]) * idy2;
+        sm[k] = v;
+    }
     __syncthreads();
     const int j = jt + c / TX, i = it + c % TX, e = (c / TX + HB) * SX + c % TX + HB;
-    const bool cell = on && j < Ny && i < Nx;
+    const bool cell = j < Ny && i < Nx;
     const bool ring = cell && G.ring(j, i), land = cell && G.land(j, i);
     float pb = 0.f, lq = 0.f, lp = 0.f, wind = 0.f;  // of cells that the parameters' terms read
     if (cell) {
@@ -179,7 +182,7 @@ __global__ void __launch_bounds__(kTileThreads* kMaxLayers)
         // the wind: every cell of layer 0, ring included; dq = 0 on land
         if (l == 0 && !land) wind = gbar[G.c(j, i)];
     }
-    if (on) spb[l * kTileThreads + c] = pb;
+    spb[l * kTileThreads + c] = pb;
     // the cotangents: a lap q, -(M Lf(a)) lap q, [bottom] -a lap psi, [top] g F / H0 (a warp is a row)
     const float a0 = cell ? sa[e] : 0.f;
     static_assert(QG_P_NU == 0 && QG_P_KAPPA == 1 && QG_P_TAU0 == 2 && QG_P_NU4 == 3, "the order of the sums");
@@ -309,10 +312,9 @@ __global__ void k_vjp_params(const double* __restrict__ pacc, int n, float* __re
     if (k < n) pbar[k] = (float)pacc[k];
 }
 
-cudaError_t launch_vjp_stencil(const VjpArgs& v, cudaStream_t s) {
-    return launch_k(k_vjp_stencil, v.n_cells * kSubX * kSubY, kTileThreads * v.max_nl, vjp_stencil_smem(v.max_nl), s, v.pdl,
-                    v.members, v.cells, v.q, v.apply_bc, v.psi, v.gbar, v.params, v.direct, v.xa, v.xa_fmt, v.xq, v.xplane,
-                    v.pacc);
+cudaError_t launch_vjp_stencil(const VjpArgs& v, int nl, const StencilTile* tiles, int n, cudaStream_t s, bool pdl) {
+    return launch_k(k_vjp_stencil, n * kSubX * kSubY, kTileThreads * nl, vjp_stencil_smem(nl), s, pdl, v.members, tiles,
+                    v.q, v.apply_bc, v.psi, v.gbar, v.params, v.direct, v.xa, v.xa_fmt, v.xq, v.xplane, v.pacc);
 }
 
 cudaError_t launch_vjp_operand(const VjpArgs& v, const float* psi_bar, cudaStream_t s) {

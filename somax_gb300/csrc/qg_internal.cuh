@@ -259,7 +259,7 @@ cudaError_t launch_residual(const MemberDev* members, const StencilTile* tiles, 
 struct VjpArgs {
     const MemberDev* members;
     const StencilTile* cells;  // 64 x 16 tiles
-    int n_cells, max_nl, n_members;
+    int n_cells, n_members;
     const float* q;       // caller packing
     int apply_bc;         // the forward zeroed the ring of q on read
     const float* psi;     // layer psi of the forward, caller packing
@@ -273,7 +273,8 @@ struct VjpArgs {
     int64_t xplane;
     bool pdl;             // programmatic dependent launch
 };
-cudaError_t launch_vjp_stencil(const VjpArgs& v, cudaStream_t s);
+// of the n tiles of members of nl layers
+cudaError_t launch_vjp_stencil(const VjpArgs& v, int nl, const StencilTile* tiles, int n, cudaStream_t s, bool pdl);
 cudaError_t launch_vjp_operand(const VjpArgs& v, const float* psi_bar, cudaStream_t s);
 cudaError_t launch_vjp_finish(const VjpArgs& v, const float* xbar, float* qbar, cudaStream_t s);
 cudaError_t launch_vjp_scatter(const VjpArgs& v, const float* xbar, float* ybar, float* const* kbar, const float* c,

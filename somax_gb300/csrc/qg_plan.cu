@@ -252,6 +252,9 @@ struct qg_plan {
     // tiles
     StencilTile* st_tiles = nullptr;
     int n_st = 0;
+    // the 64 x 16 tiles by layer count (k_vjp_stencil): those of n layers are vjp_of[n] .. vjp_of[n + 1] - 1
+    const StencilTile* vjp_tiles = nullptr;
+    int vjp_of[kMaxLayers + 2] = {};
     GemmTile* gx_tiles = nullptr;  // passes with A in x-row planes (G1, G4)
     GemmTile* gy_tiles = nullptr;  // passes with A in y-row planes (G2, G3)
     int n_gx = 0, n_gy = 0;
@@ -505,7 +508,6 @@ VjpArgs vjp_args(qg_plan* p) {
     v.members = p->md;
     v.cells = p->st_tiles_v[1];
     v.n_cells = p->n_st_v[1];
-    v.max_nl = p->max_nl;
     v.n_members = p->n_members;
     v.pacc = p->vjp_acc;
     v.xa = p->XA;
@@ -572,6 +574,21 @@ StencilArgs stencil_args(qg_plan* p, const float* params) {
 
 constexpr int kSweepRows[3] = {16, 32, 64};  // strip heights of sweep list v: kSweepRows[v % 3]
 
+// n independent launches side by side: the first on stream s (after what it waits for by programmatic
+// dependent launch), the others on side streams after an event; all joined back into s.
+template <class F>
+cudaError_t fork_join(qg_plan* p, int n, cudaStream_t s, F&& launch) {
+    cudaError_t e = cudaEventRecord(p->fork_ev, s);
+    for (int i = 0; i < n && !e; ++i) {
+        cudaStream_t ss = i == 0 ? s : p->side[(i - 1) % qg_plan::kSide];
+        if (i > 0) e = cudaStreamWaitEvent(ss, p->fork_ev, 0);
+        if (!e) e = launch(i, ss);
+        if (!e && i > 0) e = cudaEventRecord(p->join_ev[i], ss);
+    }
+    for (int i = 1; i < n && !e; ++i) e = cudaStreamWaitEvent(s, p->join_ev[i], 0);
+    return e;
+}
+
 // The multi-launch path's stencil launch: the column sweep if selected, else the tiles.
 cudaError_t launch_stencil(qg_plan* p, StencilArgs a, cudaStream_t s, bool pdl) {
     const float* planes[3] = {p->S0, p->S1, p->S2};
@@ -587,21 +604,11 @@ cudaError_t launch_stencil(qg_plan* p, StencilArgs a, cudaStream_t s, bool pdl) 
                 if (p->sw_cnt[v][g] > 0) groups[n++] = g;
             if (n <= 1 || !p->fork_ev || !p->fork_on)
                 return launch_lsweep(a, items, p->sw_cnt[v], kSweepRows[v % 3], p->sw_grid, s, pdl);
-            // fork: the first group on the stage's stream (after the last DST pass, with
-            // programmatic dependent launch), the others on side streams after an event; join
-            // them all back before the stage's next launch
-            cudaError_t e = cudaEventRecord(p->fork_ev, s);
-            for (int i = 0; i < n && !e; ++i) {
+            return fork_join(p, n, s, [&](int i, cudaStream_t ss) {
                 const int g = groups[i];
-                cudaStream_t ss = i == 0 ? s : p->side[(i - 1) % qg_plan::kSide];
-                if (i > 0) e = cudaStreamWaitEvent(ss, p->fork_ev, 0);
-                if (!e)
-                    e = launch_lsweep_group(a, items[g], p->sw_cnt[v][g], kSweepRows[v % 3], p->sw_grid[g], g, ss,
-                                            i == 0 && pdl);
-                if (!e && i > 0) e = cudaEventRecord(p->join_ev[i], ss);
-            }
-            for (int i = 1; i < n && !e; ++i) e = cudaStreamWaitEvent(s, p->join_ev[i], 0);
-            return e;
+                return launch_lsweep_group(a, items[g], p->sw_cnt[v][g], kSweepRows[v % 3], p->sw_grid[g], g, ss,
+                                           i == 0 && pdl);
+            });
         }
         // the one-layer-per-lane sweep: class 0 of each layer count
         const SweepItem* it1[kMaxLayers];
@@ -1227,6 +1234,16 @@ int qg_plan_create(const qg_member_desc* members, int n_members, const qg_option
             p->n_st_v[v] = (int)st_v[v].size();
             e = upload(p, &p->st_tiles_v[v], st_v[v]);
         }
+        p->vjp_tiles = p->st_tiles_v[1];
+        auto layers = [&](const StencilTile& t) { return members[t.member].n_layers; };
+        auto fewer = [&](const StencilTile& a, const StencilTile& b) { return layers(a) < layers(b); };
+        if (!e && !std::is_sorted(st_v[1].begin(), st_v[1].end(), fewer)) {
+            std::stable_sort(st_v[1].begin(), st_v[1].end(), fewer);
+            StencilTile* d;
+            if (!(e = upload(p, &d, st_v[1]))) p->vjp_tiles = d;
+        }
+        for (const StencilTile& t : st_v[1])
+            for (int n = layers(t) + 1; n <= kMaxLayers + 1; ++n) ++p->vjp_of[n];
         p->rw.members = p->rc.members = p->md;
         p->rw.Px = p->rc.Px = p->mh[0].Px;
         if (!e && p->rw_ok) e = rows_init(p->rw, p->rc);
@@ -1629,6 +1646,21 @@ int qg_step(qg_plan* p, float* q, const float* params, double dt, int n_steps, i
 }
 
 namespace {
+// The stencil transposes: a launch per layer count, side by side.
+cudaError_t run_vjp_stencil(qg_plan* p, const VjpArgs& v, cudaStream_t s) {
+    int nl[kMaxLayers], n = 0;
+    for (int k = 1; k <= kMaxLayers; ++k)
+        if (p->vjp_of[k] < p->vjp_of[k + 1]) nl[n++] = k;
+    auto launch = [&](int i, cudaStream_t ss) {
+        const int lo = p->vjp_of[nl[i]];
+        return launch_vjp_stencil(v, nl[i], p->vjp_tiles + lo, p->vjp_of[nl[i] + 1] - lo, ss, v.pdl && ss == s);
+    };
+    if (n > 1 && p->fork_on) return fork_join(p, n, s, launch);
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < n && !e; ++i) e = launch(i, s);
+    return e;
+}
+
 // The adjoint solve of the rhs at q for the cotangent dq_bar (its output in XC, the direct cotangent
 // of q in S2; *v: the arguments that launch_vjp_finish or _scatter needs); the parameter cotangents are
 // added to the plan's FP64 accumulators (zeroed by the caller).  psi: the layer psi of q (caller
@@ -1655,7 +1687,7 @@ cudaError_t rhs_vjp_core(qg_plan* p, const float* q, const float* params, const 
     v->gbar = dq_bar;
     v->params = params;
     v->direct = p->S2;
-    if (!e) e = timed(p, QG_K_STENCIL, s, [&] { return launch_vjp_stencil(*v, s); });
+    if (!e) e = timed(p, QG_K_STENCIL, s, [&] { return run_vjp_stencil(p, *v, s); });
     return e ? e : run_inversion(p, s);  // the adjoint solve: the inversion is self-adjoint
 }
 }  // namespace
