@@ -289,7 +289,7 @@ int qg_plan_engine(const qg_plan* plan, int* cluster_ctas, float* ms, int n);
    whose members are alike in layers (at most 5) and grid, without land, refinement or a forced
    variant; a tensor-core plan weighs it like the cluster engine (qg_options.cluster = 0) unless it
    asks for the persistent kernel.  *on = 1 when the autotuner timed it faster than the
-   pass-by-pass path; *ms (may be NULL) its time of four SSP-RK3 steps (-1 when not measured).  No
+   pass-by-pass path, or, in an FP32 plan that is not tuned, when a rule on its sizes says so; *ms (may be NULL) its time of four SSP-RK3 steps (-1 when not measured).  No
    reference counterpart. */
 int qg_plan_row_engine(const qg_plan* plan, int* on, float* ms);
 

@@ -412,6 +412,7 @@ struct RowsTable {
 int rows_quad_floats(int N);
 void rows_quad_matrix(const float* S, int N, int ld, float* out);
 bool rows_plan(int nl, int Ny, int Nx, int n_members, int n_sm, RowsArgs* r, ColsArgs* c);
+bool rows_pay(const RowsArgs& r, int n_members, int n_sm);
 cudaError_t rows_init(const RowsArgs& r, const ColsArgs& c);
 cudaError_t launch_rows(int kind, const RowsArgs& a, int n_members, cudaStream_t s, bool pdl);
 cudaError_t launch_cols(const ColsArgs& a, int n_members, cudaStream_t s, bool pdl);

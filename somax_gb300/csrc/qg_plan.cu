@@ -1405,14 +1405,14 @@ int qg_plan_create(const qg_member_desc* members, int n_members, const qg_option
     }
     if (e == cudaSuccess) {
         // the autotuner weighs the engines only when no stencil variant or tile width is forced
-        // (a forced choice asks for the pass-by-pass path); without it the row engine steps FP32
-        // plans whose members allow it
+        // (a forced choice asks for the pass-by-pass path); without it the row engine steps the FP32
+        // plans of a size that it pays for
         const bool cluster = p->cl_C > 0 && o.cluster == 0;
         if ((cluster || p->rw_ok) && o.autotune && !o.stencil && !o.gemm_tile) {
             const int r = autotune_engine(p, cluster);
             if (r != QG_OK) e = cudaErrorUnknown;
         } else {
-            p->rw_on = p->rw_ok && !tc;
+            p->rw_on = p->rw_ok && !tc && rows_pay(p->rw, n_members, std::max(p->n_sm, 1));
         }
     }
     if (e != cudaSuccess) {

@@ -167,6 +167,22 @@ bool rows_plan(int nl, int Ny, int Nx, int n_members, int n_sm, RowsArgs* r, Col
     return true;
 }
 
+// Whether a plan that is not timed steps with the row engine: by the CTAs of k_rows (an SM holds one) and
+// the multiply-adds of one (its rows' two transforms).  In one wave the engine loses only where the
+// streamed matrix and the halo rows weigh; further waves each load the matrix again, which one-layer
+// members bear longest, and tiny members not at all.  Measured over 334 plans (64^2 to 1000^2 and oblong,
+// 1 to 5 layers, 1 to 128 alike members, four SSP-RK3 steps; engine / FP32 passes): 3 x 448^2 0.99 / 1.02
+// ms, 3 x 514^2 1.45 / 1.17, 3 x 1002^2 14.9 / 5.0; members of 1 x 130^2: 16 0.45 / 0.53, 32 0.79 / 0.65;
+// of 3 x 130^2: 8 0.51 / 0.52, 16 0.88 / 0.70; of 3 x 66^2: 8 0.20 / 0.30, 16 0.37 / 0.34.  Where the rule
+// takes the engine it loses 4 % at most; where it does not, the engine gains 22 % at most.
+bool rows_pay(const RowsArgs& r, int n_members, int n_sm) {
+    const int64_t ctas = (int64_t)r.bands * n_members;
+    const int64_t work = (int64_t)(2 * r.rows + 2) * r.layers * r.x.half * r.x.NP;
+    if (ctas <= n_sm) return work <= 3200000;
+    if (r.layers == 1) return 2 * ctas <= 7 * n_sm && work <= 1050000;
+    return ctas <= 2 * n_sm && r.layers <= 4 && r.x.nch == 1 && work >= 70000;
+}
+
 // Allow the plan's kernels their shared memory (on the current device).
 cudaError_t rows_init(const RowsArgs& r, const ColsArgs& c) {
     cudaError_t e = cudaFuncSetAttribute(cols_kernel(c), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget);
