@@ -117,7 +117,8 @@ typedef struct qg_options {
                            (tensor-core precisions without refinement) */
     int autotune;       /* 1: qg_plan_create times the stencil variants and keeps the fastest */
     int stencil;        /* 0: autotuner's choice; QG_STENCIL_* + 1: run that variant */
-    int gemm_tile;      /* 0: autotuner's choice; 144, 80, 48, 32 or 16: that tensor-core tile width */
+    int gemm_tile;      /* 0: autotuner's choice; 144, 80, 48, 32 or 16, without the persistent kernel also
+                           176, 208 or 256: that tensor-core tile width */
     int cluster;        /* cluster-resident stepping of small members (qg_step with Heun / SSP-RK3:
                            one thread-block cluster per member runs every stage of every step in
                            one launch, FP32 DST passes on the CUDA cores, state in shared memory):
