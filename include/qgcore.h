@@ -275,9 +275,14 @@ int qg_kernel_stats(qg_plan* plan, int kclass, double* total_ms, int64_t* launch
    the autotuner's time of one stage with variant k in ms (-1 when not measured). */
 int qg_plan_tuning(const qg_plan* plan, int* variant, float* ms, int n);
 /* The tensor-core DST passes' output tile width the autotuner kept (144, 80, 48, 32, 16, 176,
-   208 or 256 columns; 64 for the FP32 CUDA-core passes) and the time of the four passes it
-   measured with each width in ms (ms[0..7] in that order; -1 when not measured). */
+   208 or 256 columns; for the FP32 CUDA-core passes the width that the plan's sizes chose, see
+   qg_plan_pass_tile) and the time of the four passes it measured with each tensor-core width in ms
+   (ms[0..7] in that order; -1 when not measured). */
 int qg_plan_gemm_tuning(const qg_plan* plan, int* tile_n, float* ms, int n);
+/* Rows and columns of a DST pass's output tile: 128 x the width above on the tensor cores; 64 x 96,
+   64 x 48, 32 x 48 or 16 x 16 for the FP32 passes.  Either pointer may be NULL.  No reference
+   counterpart. */
+int qg_plan_pass_tile(const qg_plan* plan, int* rows, int* cols);
 /* The stepping engine qg_step uses for Heun / SSP-RK3: *cluster_ctas = the CTAs of one
    member's cluster when the cluster-resident engine runs (all members alike in layers and
    grid, unmasked, small enough for one cluster's shared memory), else 0; ms[0], ms[1] (n >= 2)
@@ -290,8 +295,9 @@ int qg_plan_engine(const qg_plan* plan, int* cluster_ctas, float* ms, int n);
    whose members are alike in layers (at most 5) and grid, without land, refinement or a forced
    variant; a tensor-core plan weighs it like the cluster engine (qg_options.cluster = 0) unless it
    asks for the persistent kernel.  *on = 1 when the autotuner timed it faster than the
-   pass-by-pass path, or, in an FP32 plan that is not tuned, when a rule on its sizes says so; *ms (may be NULL) its time of four SSP-RK3 steps (-1 when not measured).  No
-   reference counterpart. */
+   pass-by-pass path, or, in an FP32 plan that is not tuned, when a rule on its sizes says so;
+   *ms (may be NULL) its time of four SSP-RK3 steps (-1 when not measured).  No reference
+   counterpart. */
 int qg_plan_row_engine(const qg_plan* plan, int* on, float* ms);
 
 /* dst (device) = n host floats, in stream order without waiting for the stream: they travel as

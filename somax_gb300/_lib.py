@@ -98,6 +98,7 @@ def lib() -> C.CDLL:
         "qg_kernel_stats": (C.c_int, [vp, C.c_int, C.POINTER(C.c_double), C.POINTER(i64)]),
         "qg_plan_tuning": (C.c_int, [vp, C.POINTER(C.c_int), C.POINTER(C.c_float), C.c_int]),
         "qg_plan_gemm_tuning": (C.c_int, [vp, C.POINTER(C.c_int), C.POINTER(C.c_float), C.c_int]),
+        "qg_plan_pass_tile": (C.c_int, [vp, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
         "qg_plan_engine": (C.c_int, [vp, C.POINTER(C.c_int), C.POINTER(C.c_float), C.c_int]),
         "qg_plan_row_engine": (C.c_int, [vp, C.POINTER(C.c_int), C.POINTER(C.c_float)]),
         "qg_write": (C.c_int, [vp, vp, i64, vp]),

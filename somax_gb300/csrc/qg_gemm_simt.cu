@@ -207,6 +207,8 @@ static_assert(Shape0::SMEM <= 48 * 1024 && Shape1::SMEM <= 48 * 1024 && Shape2::
 
 }  // namespace
 
+int simt_tile_rows(int shape) { return kShapes[shape].bm; }
+int simt_tile_cols(int shape) { return 2 * kShapes[shape].bn; }
 int simt_row_tiles(int shape, int rows) { return (rows + kShapes[shape].bm - 1) / kShapes[shape].bm; }
 int simt_col_tiles(int shape, int n) { return ((n + 1) / 2 + kShapes[shape].bn - 1) / kShapes[shape].bn; }
 

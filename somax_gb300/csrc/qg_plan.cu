@@ -1911,8 +1911,16 @@ int qg_plan_tuning(const qg_plan* p, int* variant, float* ms, int n) {
 
 int qg_plan_gemm_tuning(const qg_plan* p, int* tile_n, float* ms, int n) {
     if (!p) return QG_ERR_NULL;
-    if (tile_n) *tile_n = p->opts.dst_precision == QG_DST_FP32 ? 64 : kGemmBN[p->bn_sel];
+    if (tile_n) qg_plan_pass_tile(p, nullptr, tile_n);
     for (int k = 0; ms && k < n && k < kNumBN; ++k) ms[k] = p->tune_gemm_ms[k];
+    return QG_OK;
+}
+
+int qg_plan_pass_tile(const qg_plan* p, int* rows, int* cols) {
+    if (!p) return QG_ERR_NULL;
+    const bool fp32 = p->opts.dst_precision == QG_DST_FP32;
+    if (rows) *rows = fp32 ? simt_tile_rows(p->simt_sel) : 128;
+    if (cols) *cols = fp32 ? simt_tile_cols(p->simt_sel) : kGemmBN[p->bn_sel];
     return QG_OK;
 }
 

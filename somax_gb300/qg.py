@@ -446,9 +446,11 @@ class Plan:
         bn = C.c_int()
         gms = (C.c_float * 8)()
         check(self._L.qg_plan_gemm_tuning(self._h, C.byref(bn), gms, len(gms)), "qg_plan_gemm_tuning")
+        rows = C.c_int()
+        check(self._L.qg_plan_pass_tile(self._h, C.byref(rows), None), "qg_plan_pass_tile")
         return {"stencil": self.STENCIL_VARIANTS[v.value],
                 "ms": {name: round(float(t), 5) for name, t in zip(self.STENCIL_VARIANTS, ms)},
-                "gemm_tile_n": bn.value,
+                "gemm_tile_n": bn.value, "gemm_tile_rows": rows.value,
                 "gemm_ms": {w: round(float(t), 5) for w, t in zip((144, 80, 48, 32, 16, 176, 208, 256), gms)}}
 
     def engine(self) -> dict:
