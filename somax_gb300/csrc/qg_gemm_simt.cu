@@ -39,8 +39,7 @@ struct Shape {
 using Shape0 = Shape<4, 6, 8, 16, 3>;  // 64 x 48
 using Shape1 = Shape<4, 3, 8, 16, 4>;  // 64 x 24
 using Shape2 = Shape<2, 3, 8, 16, 5>;  // 32 x 24
-using Shape3 = Shape<2, 1, 8, 16, 5>;  // 32 x 8
-using Shape4 = Shape<1, 1, 8, 16, 6>;  // 16 x 8
+using Shape3 = Shape<1, 1, 8, 16, 6>;  // 16 x 8
 
 struct PassGeom {
     int Mb, K, Mtot, lda, ldo;
@@ -199,10 +198,9 @@ template <class S>
 constexpr ShapeInfo info() {
     return {S::BM, S::BN, S::NT, S::SMEM, Passes<S>::k};
 }
-const ShapeInfo kShapes[kSimtShapes] = {info<Shape0>(), info<Shape1>(), info<Shape2>(), info<Shape3>(),
-                                        info<Shape4>()};
+const ShapeInfo kShapes[kSimtShapes] = {info<Shape0>(), info<Shape1>(), info<Shape2>(), info<Shape3>()};
 static_assert(Shape0::SMEM <= 48 * 1024 && Shape1::SMEM <= 48 * 1024 && Shape2::SMEM <= 48 * 1024 &&
-                  Shape3::SMEM <= 48 * 1024 && Shape4::SMEM <= 48 * 1024,
+                  Shape3::SMEM <= 48 * 1024,
               "no opt-in to more shared memory");
 
 }  // namespace
@@ -221,7 +219,7 @@ int simt_col_tiles(int shape, int n) { return ((n + 1) / 2 + kShapes[shape].bn -
 // 5-layer 502 x 702 44.3 / 50.0 / 108 us (64 x 24), 3-layer 1026^2 102 / 128 / 337 us (64 x 48);
 // each figure holds ~5 us of event overhead.
 int simt_shape(const int64_t (&tiles)[kSimtShapes], int n_sm) {
-    constexpr int weight[kSimtShapes] = {10, 12, 13, 20, 20};
+    constexpr int weight[kSimtShapes] = {10, 12, 13, 20};
     int best = 0;
     int64_t least = 0;
     for (int k = 0; k < kSimtShapes; ++k) {

@@ -346,7 +346,7 @@ cudaError_t gemm_tc_encode(const MemberDev& M, int pass, const void* a_plane, in
 // FP32 CUDA-core passes (qg_gemm_simt.cu): tile shapes, from the largest to the smallest; a
 // pass over members with N columns has simt_row_tiles(shape, rows) x simt_col_tiles(shape, N)
 // tiles of one, which forms simt_tile_rows x simt_tile_cols outputs.
-constexpr int kSimtShapes = 5;
+constexpr int kSimtShapes = 4;
 int simt_tile_rows(int shape);
 int simt_tile_cols(int shape);
 int simt_row_tiles(int shape, int rows);
