@@ -407,6 +407,10 @@ int64_t qg_swm_step_vjp_workspace(const qg_swm_plan* plan, int scheme);
    that of y_start on return, params_bar the parameter cotangents summed over the k steps.
    Replayed as one captured graph while its pointers, dt, k and the scheme repeat. */
 int64_t qg_swm_segment_vjp_workspace(const qg_swm_plan* plan, int scheme, int k);
+/* The most bytes of stage inputs a segment keeps (default 2^30): within them the workspace holds every
+   step's, and each step's stages run once; beyond them (0: always) the reverse sweep runs them again in a
+   workspace of one step's.  Asks for the workspace size again.  No reference counterpart. */
+int qg_swm_set_kept_inputs(qg_swm_plan* plan, int64_t bytes);
 int qg_swm_segment_vjp(qg_swm_plan* plan, const float* y_start, const float* params, double dt, int k, int scheme,
                        float* y_bar, float* params_bar, float* work, void* stream);
 int qg_swm_step_vjp(qg_swm_plan* plan, const float* y0, const float* params, double dt, int scheme, float* y_bar,

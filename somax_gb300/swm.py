@@ -212,16 +212,7 @@ class SwmPlan:
         self._check(y_start, "state")
         self._check(g, "cotangent")
         params = self._params(params)
-        bufs = getattr(self, "_seg_bufs", {})
-        self._seg_bufs = bufs
-        key = (scheme, int(k))
-        need = int(self._L.qg_swm_segment_vjp_workspace(self._h, _SCHEMES[scheme], int(k)))
-        b = bufs.get(key)
-        if b is None or b[3].device != y_start.device:
-            b = (torch.empty_like(y_start), torch.empty_like(y_start),
-                 torch.empty(3, dtype=torch.float32, device=y_start.device),
-                 torch.empty(need, dtype=torch.float32, device=y_start.device))
-            bufs[key] = b
+        b = self._segment_buffers(y_start, scheme, int(k))
         yin, yb, pb, work = b
         yin.copy_(y_start)
         yb.copy_(g)
@@ -230,6 +221,37 @@ class SwmPlan:
                                          C.c_void_p(pb.data_ptr()), C.c_void_p(work.data_ptr()),
                                          _stream_handle(y_start.device)), "qg_swm_segment_vjp")
         return yb.clone(), pb.clone()
+
+    def _segment_buffers(self, y: torch.Tensor, scheme: str, k: int):
+        """Staged state, cotangent, parameter cotangents and workspace of ``segment_vjp``: one set for every
+        segment of the plan, its workspace as large as the largest of them.  Where the device cannot
+        hold the stage inputs that a segment would keep, the plan keeps none from then on."""
+        def size():
+            return int(self._L.qg_swm_segment_vjp_workspace(self._h, _SCHEMES[scheme], k))
+
+        def allocate():
+            return [torch.empty(n, dtype=torch.float32, device=y.device) for n in (y.numel(), y.numel(), 3, size())]
+
+        stream = torch.cuda.current_stream(y.device)
+        b, own = getattr(self, "_seg_bufs", None) or (None, None)
+        if b is None or b[3].numel() < size():
+            b = self._seg_bufs = None  # first, so that their memory can serve the larger ones
+            try:
+                b = allocate()
+            except torch.cuda.OutOfMemoryError:
+                self.set_kept_inputs(0)
+                b = allocate()
+            own, self._seg_bufs = stream, (b, stream)
+        if stream != own:
+            for t in b:  # when they are replaced, this stream may still read them
+                t.record_stream(stream)
+        return b
+
+    def set_kept_inputs(self, nbytes: int):
+        """The most bytes of stage inputs that ``segment_vjp`` keeps for a segment (1 GiB unless set; 0: none,
+        each step's stages run twice, in a smaller workspace); drops the buffers of earlier segments."""
+        check(self._L.qg_swm_set_kept_inputs(self._h, int(nbytes)), "qg_swm_set_kept_inputs")
+        self._seg_bufs = None
 
     def field_stats(self, x: torch.Tensor) -> torch.Tensor:
         """(min, mean, max) over the finite entries of the float32 CUDA tensor x and the count of
