@@ -41,17 +41,8 @@ constexpr int TX = 32, TY = 4, HB = 2;  // tile and halo (the biharmonic reaches
 constexpr int SX = TX + 2 * HB, SY = TY + 2 * HB;
 constexpr int NT = 256;
 
-__device__ __forceinline__ bool on_ring(int j, int i, int Ny, int Nx) {
-    return j == 0 || i == 0 || j == Ny - 1 || i == Nx - 1;
-}
 __device__ __forceinline__ bool interior(int j, int i, int Ny, int Nx) {
     return j > 0 && i > 0 && j < Ny - 1 && i < Nx - 1;
-}
-__device__ __forceinline__ int64_t cidx(const MemberDev& M, int l, int j, int i) {
-    return M.off_state + ((int64_t)l * M.Ny + j) * M.Nx + i;
-}
-__device__ __forceinline__ int64_t xidx(const MemberDev& M, int l, int j, int i) {
-    return M.off_x + ((int64_t)l * M.Ny + j) * M.Px + i;
 }
 
 }  // namespace
