@@ -123,7 +123,9 @@ typedef struct qg_options {
                            one thread-block cluster per member runs every stage of every step in
                            one launch, FP32 DST passes on the CUDA cores, state in shared memory):
                            0: used when the autotuner times it faster than the multi-launch path,
-                           1: used whenever the members allow it, 2: never */
+                           1: used whenever the members allow it, 2: never.  In a tensor-core plan
+                           1 and 2 also keep the row engine out (see qg_plan_row_engine): with 2
+                           every step runs the passes of the plan's own precision */
 } qg_options;
 
 typedef struct qg_plan qg_plan;

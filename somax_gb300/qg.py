@@ -225,7 +225,10 @@ class Plan:
                  device=None, persistent=True, autotune=True, stencil=None, gemm_tile=None, cluster=None):
         """``cluster``: cluster-resident stepping of small members (``step`` with Heun / SSP-RK3 in
         one launch per call): None = when the autotuner times it faster, True = whenever the
-        members allow it, False = never."""
+        members allow it, False = never.  The cluster and the row engine compute in FP32; with False a
+        tensor-core plan steps with the passes of its own precision only.  ``persistent``: the
+        persistent kernel of a tensor-core plan, which the row engine is not weighed against;
+        ``persistent=False`` is the faster choice."""
         if not torch.cuda.is_available():
             raise RuntimeError("somax_gb300 needs a CUDA device (no CPU fallback)")
         d = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
